@@ -246,3 +246,73 @@ def tolerance(case):
     if case["kind"] in ("bf16", "f16"):
         return {"rel": 4e-3, "max": 0.08}
     return {"rel": 2e-3, "max": 0.16}
+
+
+# ---------------------------------------------------------------------------
+# the same answers in 64 bits
+# ---------------------------------------------------------------------------
+def _exact_weight(kind, w, s):
+    """One expert's weight [N, K] as the values its codes and scales stand for."""
+    if kind in ("bf16", "f16"):
+        return w.double()
+    if kind == "fp8_block":
+        return w.double() * s.double().repeat_interleave(128, 0).repeat_interleave(128, 1)
+    if kind == "int8_channel":
+        return w.double() * s.double()[:, None]
+    if kind == "mxfp4":
+        table = torch.tensor((0, .5, 1, 1.5, 2, 3, 4, 6), dtype=torch.float64, device=w.device)
+        code = torch.stack((w & 15, w >> 4), -1).flatten(-2).long()
+        w = table[code & 7] * torch.where(code & 8 != 0, -1.0, 1.0)
+    return w.double() * torch.exp2(s.double() - 127).repeat_interleave(32, 1)
+
+
+def _exact_rows(kind, v):
+    """Activations [m, K] after the recipe's quantiser (which is part of what the layer computes)."""
+    if kind in ("bf16", "f16"):
+        return v
+    group = {"fp8_block": 128, "int8_channel": v.shape[1], "mxfp8": 32, "mxfp4": 128}[kind]
+    y = v.view(v.shape[0], -1, group)
+    amax = y.abs().amax(-1, keepdim=True).clamp_min(1e-10)
+    if kind == "int8_channel":
+        s = amax / 127.0
+        return ((y / s).round() * s).view(v.shape)
+    s = amax / 448.0
+    if kind.startswith("mx"):
+        s = torch.exp2(torch.ceil(torch.log2(s)))
+    return ((y / s).float().to(FP8).double() * s).view(v.shape)
+
+
+def exact(case, seed):
+    state = prepare(case, seed)
+    x = state["x"]
+    if case["op"] == "dense":
+        xd = (x.double().view(case["M"], -1, 128) * state["xs"].double()[..., None]).flatten(1)
+        return xd @ _exact_weight("fp8_block", state["w"], state["ws"]).t()
+    kind, kw = case["kind"], state["kw"]
+    if case["router"]:
+        scores, ids = torch.softmax(state["logits"].double(), -1).topk(case["K"], -1)
+        weights = scores / scores.sum(-1, keepdim=True)
+    else:
+        weights, ids = state["weights"].double(), state["ids"].long()
+    if "expert_map" in kw:
+        ids = kw["expert_map"].long()[ids]
+    rows = _exact_rows(kind, x.double())
+    out = torch.zeros_like(rows)
+    for e in range(state["w1"].shape[0]):
+        token, slot = (ids == e).nonzero(as_tuple=True)
+        if not token.numel():
+            continue
+        s1, s2 = (kw[n][e] if n in kw else None for n in ("w1_scale", "w2_scale"))
+        g = rows[token] @ _exact_weight(kind, state["w1"][e], s1).t()
+        if case.get("clamp"):
+            gate, up = (g + kw["b1"][e].double()).chunk(2, -1)
+            gate, up = gate.clamp(max=7.0), up.clamp(-7.0, 7.0)
+            act = gate * torch.sigmoid(1.702 * gate) * (up + 1)
+        else:
+            gate, up = g.chunk(2, -1)
+            act = gate * torch.sigmoid(gate) * up
+        y = _exact_rows(kind, act) @ _exact_weight(kind, state["w2"][e], s2).t()
+        if case.get("clamp"):
+            y = y + kw["b2"][e].double()
+        out.index_add_(0, token, y * weights[token, slot][:, None])
+    return (out, weights, None) if case["router"] else out

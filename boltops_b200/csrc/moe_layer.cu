@@ -128,7 +128,7 @@ extern "C" int bolt_moe_layer_kernel_count(const bolt_layer_args* a) {
   Plan p;
   if (check_args(a) != BOLT_OK || make_plan(a, p) != BOLT_OK) return -1;
   if (a->num_tokens == 0) return 0;
-  const int sort = p.sort_ws_bytes <= 16 ? 1 : 3;
+  const int sort = p.sort_ws_bytes <= 16 ? 1 : 2;
   const int place = p.block ? 1 : (p.quant ? 2 : (p.gather ? 0 : 1));
   return sort + place + 2 + (p.quant && !p.block ? 1 : 0) + 1;
 }

@@ -40,8 +40,8 @@ def _require_cuda(*tensors):
 
 
 def sort_launches(lib, m: int, topk: int, num_experts: int) -> int:
-    """Kernels one sort launches: one CTA does everything for small inputs, three kernels else."""
-    return 1 if lib.bolt_moe_sort_workspace_bytes(m, topk, num_experts) <= 16 else 3
+    """Kernels one sort launches: one for small inputs, two else."""
+    return 1 if lib.bolt_moe_sort_workspace_bytes(m, topk, num_experts) <= 16 else 2
 
 
 def ceil_to(x: int, m: int) -> int:

@@ -39,10 +39,16 @@ using namespace tc;
 
 constexpr int kThreads = 384;
 constexpr int kMaxDevices = 64;
-// shared-memory operand stages: the block-scaled kinds spend ~950 cycles per K block (three
-// stages cover the load latency, and the space goes to bulk-store slots); the others stream a
-// K block every ~500 cycles and need four
-constexpr int stages_of(bool block_scaled) { return block_scaled ? 3 : 4; }
+// Shared-memory operand stages against bulk-store slots.  The block-scaled kinds spend ~950 cycles
+// per K block, three stages cover the load latency, and the space goes to the slots.  The other
+// 8-bit kinds stream a K block every ~500 cycles; their down projection runs a short reduction,
+// so that the stores are the longer half of a tile, and takes the same division (Qwen3-30B int8,
+// 16384 tokens, K = 768: 284 us with one slot per warp, 232 us with four).  Their gated GEMM and the
+// 16-bit kinds keep four stages (same layer, K = 2048: 366 us against 381 us with three).
+constexpr bool more_slots(int opk, bool block_scaled, int epi) {
+  return block_scaled || (opk != OP_F16 && epi == BOLT_EPI_STORE);
+}
+constexpr int stages_of(bool slots) { return slots ? 3 : 4; }
 constexpr int kBM = 128;
 constexpr int kAccCols = 256;           // accumulator columns per tile
 constexpr int kHalfCols = 128;          // columns of one independently scheduled half
@@ -52,21 +58,21 @@ constexpr int kBBytes = kAccCols * 128; // 32 KiB
 constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kScaleSlots = 8;           // ring of per-K-block activation-scale rows (512 B each)
 constexpr int kOutSlotBytes = 32 * 64;    // one 32-row x 64-byte block as a bulk store reads it
-// per epilogue warp: block-scaled kinds one slot per 32-column chunk of a tile, the others one
-// slot that is reclaimed chunk by chunk (their epilogue overlaps the next tile's MMAs anyway)
-constexpr int out_slots_of(bool block_scaled) { return block_scaled ? 4 : 1; }
-constexpr int out_stage_bytes_of(bool block_scaled) { return block_scaled ? 4 * kOutSlotBytes : 2560; }
+// per epilogue warp: one slot per 32-column chunk of a tile, or one slot that is reclaimed chunk
+// by chunk
+constexpr int out_slots_of(bool slots) { return slots ? 4 : 1; }
+constexpr int out_stage_bytes_of(bool slots) { return slots ? 4 * kOutSlotBytes : 2560; }
 // (the padded 32 x 80 B layout of the staged fallback path fits in either)
-constexpr int smem_bytes_of(bool block_scaled) {
-  return stages_of(block_scaled) * kStageBytes + 4096 + kScaleSlots * 512 +
-         8 * out_stage_bytes_of(block_scaled) + 1024;  // +1024 alignment slack
+constexpr int smem_bytes_of(bool slots) {
+  return stages_of(slots) * kStageBytes + 4096 + kScaleSlots * 512 +
+         8 * out_stage_bytes_of(slots) + 1024;  // +1024 alignment slack
 }
 // CTA pairs stage half of the B tile per CTA: 32 KiB per stage, so more stages fit
 constexpr int kPairStageBytes = kABytes + kBBytes / 2;
-constexpr int pair_stages_of(bool block_scaled) { return block_scaled ? 4 : 5; }
-constexpr int pair_smem_bytes_of(bool block_scaled) {
-  return pair_stages_of(block_scaled) * kPairStageBytes + 4096 + kScaleSlots * 512 +
-         8 * out_stage_bytes_of(block_scaled) + 1024;
+constexpr int pair_stages_of(bool slots) { return slots ? 4 : 5; }
+constexpr int pair_smem_bytes_of(bool slots) {
+  return pair_stages_of(slots) * kPairStageBytes + 4096 + kScaleSlots * 512 +
+         8 * out_stage_bytes_of(slots) + 1024;
 }
 
 
@@ -344,7 +350,51 @@ struct RowMeta {
   int sid;
   float rw;
   float a_s;  // channel kinds: row scale
+  float col_s, col_b;  // kinds that sum over K in TMEM: scale and bias of accumulator column (thread
+                       // index in the half)
 };
+
+// Barrier of the 128 epilogue threads of half h; tells whether any of them is in trouble.
+__device__ __forceinline__ bool half_any(int h, bool bad) {
+  int r;
+  asm volatile(
+      "{\n.reg .pred p, q;\nsetp.ne.b32 p, %1, 0;\n"
+      "barrier.cta.red.or.pred q, %2, 128, p;\nselp.b32 %0, 1, 0, q;\n}\n"
+      : "=r"(r)
+      : "r"((int)bad), "r"(1 + h)
+      : "memory");
+  return r != 0;
+}
+
+// 32 accumulator columns -> results: times the row's and the columns' scales (CHANNEL), plus bias
+// (one rounding for the last product and the sum), times the router weight.
+template <int OPK, bool CHANNEL>
+__device__ __forceinline__ void scale_columns(const uint32_t (&raw)[32], float (&v)[32], float a_s,
+                                              const float* col_s, const float* col_b, bool has_bias,
+                                              bool has_rw, float rw) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 4) {
+    float4 s = make_float4(1.f, 1.f, 1.f, 1.f);
+    if (CHANNEL) s = *reinterpret_cast<const float4*>(col_s + j);
+    const float sc[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[j + i] = acc_to_f32<OPK>(raw[j + i]);
+    if (has_bias) {
+      const float4 b = *reinterpret_cast<const float4*>(col_b + j);
+      const float bi[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        v[j + i] = CHANNEL ? fmaf(v[j + i] * a_s, sc[i], bi[i]) : v[j + i] + bi[i];
+    } else if (CHANNEL) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[j + i] = v[j + i] * a_s * sc[i];
+    }
+    if (has_rw) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[j + i] *= rw;
+    }
+  }
+}
 
 // ---------------------------------------------------------------------------
 // Kernel
@@ -367,11 +417,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 k_grouped_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                const __grid_constant__ CUtensorMap tma_c, const GemmParams p) {
   constexpr bool GATED = EPI != BOLT_EPI_STORE;
+  constexpr bool MORE_SLOTS = more_slots(OPK, BS, EPI);
   constexpr int kBKElems = OPK == OP_F16 ? 64 : 128;
   constexpr bool CHANNEL = (OPK != OP_F16) && !BS;
-  constexpr int kStages = PAIR ? pair_stages_of(BS) : stages_of(BS);
+  constexpr int kStages = PAIR ? pair_stages_of(MORE_SLOTS) : stages_of(MORE_SLOTS);
   constexpr int kStageStride = PAIR ? kPairStageBytes : kStageBytes;
-  constexpr int kSlots = out_slots_of(BS);
+  constexpr int kSlots = out_slots_of(MORE_SLOTS);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -689,9 +740,10 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
     const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * q) << 16) + h * kHalfCols;
     const bool has_ids = p.sorted_ids != nullptr;
     const bool has_rw = p.mul_routed_weight && p.sorted_weights != nullptr;
-    uint8_t* out_stage = ctrl + 4096 + kScaleSlots * 512 + (warp - 4) * out_stage_bytes_of(BS);
+    uint8_t* out_stage = ctrl + 4096 + kScaleSlots * 512 + (warp - 4) * out_stage_bytes_of(MORE_SLOTS);
     int t = 0;
     uint32_t tph = 0, xph = 0, kbi = 0;
+    int colbuf = 0;
     bool ok = true;
 
     // coordinates and per-row metadata of a work item (an idle CTA of a pair mirrors rank 0's
@@ -703,6 +755,20 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       m.sid = has_ids ? p.sorted_ids[r] : 0;
       m.rw = has_rw ? p.sorted_weights[r] : 1.0f;
       m.a_s = CHANNEL ? p.a_scale[r] : 1.0f;
+      m.col_s = 1.0f;
+      m.col_b = 0.0f;
+      if (!BS && (CHANNEL || p.bias != nullptr) && m.expert >= 0 && m.expert < p.num_experts) {
+        int col;
+        if (GATED) {
+          col = min(c.n_blk * 128 + 64 * h + (row_in_tile & 63), p.n_half - 1) +
+                (row_in_tile < 64 ? 0 : p.n_half);
+        } else {
+          col = min(c.n_blk * 256 + 128 * h + row_in_tile, p.n - 1);
+        }
+        const int64_t at = (int64_t)m.expert * p.n + col;
+        if (CHANNEL) m.col_s = __ldg(p.b_scale + at);
+        if (p.bias != nullptr) m.col_b = load_bias(p.bias, p.bias_dtype, at);
+      }
       return m;
     };
     // hand a TMEM stage back to the MMA issuer (of the pair: the even CTA's barrier)
@@ -771,7 +837,21 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       const int ocol = GATED ? tc.n_blk * 128 + 64 * h : tc.n_blk * 256 + 128 * h;
 
       if (!BS) {
+        // Scales and biases of the half's 128 accumulator columns go to shared memory, one column per
+        // thread (loaded a tile ahead), and come back as broadcasts: a load of its own per
+        // column and row was most of this epilogue.  Two buffers, one barrier per tile.
+        const bool has_bias = p.bias != nullptr;
+        float* col_s = as_ring + (colbuf * 2 + h) * kHalfCols;
+        float* col_b = col_s + 4 * kHalfCols;
+        if (CHANNEL || has_bias) {
+          col_s[row_in_tile] = cur.col_s;
+          col_b[row_in_tile] = cur.col_b;
+          colbuf ^= 1;
+        }
         ok = mbar_wait(bar_tfull + 8 * t, tph, abort_flag, p.status, 4);
+        if (CHANNEL || has_bias) {
+          if (half_any(h, !ok)) ok = false;
+        }
         if (!ok) break;
         tc_fence_after();
         if (lane == 0) bulk_wait_read();   // the previous tile's bulk stores have left the slots
@@ -779,31 +859,14 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         const uint32_t tbase = lane_addr + t * kAccCols;
         const float a_s = cur.a_s;
         if (!GATED) {
-          const int ncols = p.n;
 #pragma unroll 1
           for (int i = 0; i < 4; ++i) {
             uint32_t raw[32];
             tmem_ld32(tbase + 32 * i, raw);
             tmem_ld_wait();
-            const int col0 = ocol + 32 * i;
             float v[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = acc_to_f32<OPK>(raw[j]);
-            if (CHANNEL) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                v[j] = v[j] * a_s * __ldg(p.b_scale + brow + min(col0 + j, ncols - 1));
-            }
-            if (p.bias) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                v[j] += load_bias(p.bias, p.bias_dtype, brow + min(col0 + j, ncols - 1));
-            }
-            if (has_rw) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] *= rw;
-            }
-            store_chunk<kSlots>(out_stage, i, p, &tma_c, tile_row0, row_off, col0, ncols, live, lane, v);
+            scale_columns<OPK, CHANNEL>(raw, v, a_s, col_s + 32 * i, col_b + 32 * i, has_bias, has_rw, rw);
+            store_chunk<kSlots>(out_stage, i, p, &tma_c, tile_row0, row_off, ocol + 32 * i, p.n, live, lane, v);
           }
         } else {
 #pragma unroll 1
@@ -812,38 +875,16 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
             tmem_ld32(tbase + 32 * i, rg);
             tmem_ld32(tbase + 64 + 32 * i, ru);
             tmem_ld_wait();
-            const int col0 = ocol + 32 * i;
             float g[32], u[32];
+            scale_columns<OPK, CHANNEL>(rg, g, a_s, col_s + 32 * i, col_b + 32 * i, has_bias, has_rw, rw);
+            scale_columns<OPK, CHANNEL>(ru, u, a_s, col_s + 64 + 32 * i, col_b + 64 + 32 * i, has_bias,
+                                        has_rw, rw);
+            if (!live) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              g[j] = live ? acc_to_f32<OPK>(rg[j]) : 0.f;
-              u[j] = live ? acc_to_f32<OPK>(ru[j]) : 0.f;
-            }
-            if (CHANNEL) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const int col = min(col0 + j, p.n_half - 1);
-                g[j] = g[j] * a_s * __ldg(p.b_scale + brow + col);
-                u[j] = u[j] * a_s * __ldg(p.b_scale + brow + p.n_half + col);
-              }
-            }
-            if (p.bias) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const int col = min(col0 + j, p.n_half - 1);
-                g[j] += load_bias(p.bias, p.bias_dtype, brow + col);
-                u[j] += load_bias(p.bias, p.bias_dtype, brow + p.n_half + col);
-              }
-            }
-            if (has_rw) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                g[j] *= rw;
-                u[j] *= rw;
-              }
+              for (int j = 0; j < 32; ++j) g[j] = u[j] = 0.f;
             }
             silu_mul32_dyn(g, u, p.mid_dtype);
-            store_chunk<kSlots>(out_stage, i, p, &tma_c, tile_row0, row_off, col0, p.n_half, wr, lane, g);
+            store_chunk<kSlots>(out_stage, i, p, &tma_c, tile_row0, row_off, ocol + 32 * i, p.n_half, wr, lane, g);
           }
         }
         tc_fence_before();
@@ -1477,7 +1518,8 @@ template <int OPK, bool BS, int EPI, bool PAIR>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc,
            const GemmParams& p, int grid, cudaStream_t st) {
   auto kfn = k_grouped_gemm<OPK, BS, EPI, PAIR>;
-  constexpr int smem = PAIR ? pair_smem_bytes_of(BS) : smem_bytes_of(BS);
+  constexpr bool slots = more_slots(OPK, BS, EPI);
+  constexpr int smem = PAIR ? pair_smem_bytes_of(slots) : smem_bytes_of(slots);
   static std::atomic<bool> configured[kMaxDevices];
   // warps 0-3 drop to 56 registers, the eight epilogue warps rise to 224
   const int rc = configure_kernel(kfn, smem, configured, 128, 56, 256, 224);

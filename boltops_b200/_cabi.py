@@ -26,7 +26,7 @@ GEMM_BF16, GEMM_F16, GEMM_FP8_BLOCK, GEMM_INT8_CHANNEL, GEMM_FP8_CHANNEL, GEMM_I
 # enum bolt_gemm_epilogue
 EPI_STORE, EPI_SILU_MUL, EPI_SILU_MUL_QUANT = range(3)
 # enum bolt_gemm_schedule, BOLT_PAIR_SEGMENT_ROWS
-SCHEDULE_ROW_TILES, SCHEDULE_TILE_PAIRS = range(2)
+SCHEDULE_ROW_TILES, SCHEDULE_TILE_PAIRS, SCHEDULE_STREAM = range(3)
 PAIR_SEGMENT_ROWS = 256
 
 _DTYPES = {
@@ -78,7 +78,7 @@ class LayerArgs(C.Structure):
         ("topk_weights", C.c_void_p), ("topk_ids", C.c_void_p), ("expert_mask", C.c_void_p),
         ("routed_scaling_factor", C.c_float),
         ("out", C.c_void_p), ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t),
-        ("status", C.c_void_p),
+        ("status", C.c_void_p), ("schedule", C.c_int),
     ]
 
 

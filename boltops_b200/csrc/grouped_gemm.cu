@@ -31,6 +31,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "stream_gemm.cuh"
 #include "tc_ptx.cuh"
 
 namespace bolt {
@@ -38,7 +39,6 @@ namespace {
 using namespace tc;
 
 constexpr int kThreads = 384;
-constexpr int kMaxDevices = 64;
 // Shared-memory operand stages against bulk-store slots.  The block-scaled kinds spend ~950 cycles
 // per K block, three stages cover the load latency, and the space goes to the slots.  The other
 // 8-bit kinds stream a K block every ~500 cycles; their down projection runs a short reduction,
@@ -1487,33 +1487,6 @@ EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// One-time set-up of a kernel on the CURRENT device (`done` has one slot per device ordinal):
-// the dynamic shared-memory opt-in is a per-device attribute, and a kernel that re-splits its
-// registers with setmaxnreg must have been compiled to a register count from which the split
-// balances -- `setmaxnreg.inc` only gets registers that `setmaxnreg.dec` released in the same
-// CTA and waits forever otherwise, so an unbalanced split is refused here instead of launched.
-// dec_threads drop to dec_regs, inc_threads rise to inc_regs (0 threads: no split).
-template <typename KernelT>
-int configure_kernel(KernelT kfn, int smem_bytes, std::atomic<bool>* done, int dec_threads,
-                     int dec_regs, int inc_threads, int inc_regs) {
-  int dev = 0;
-  BOLT_CUDA(cudaGetDevice(&dev));
-  BOLT_REQUIRE(dev >= 0 && dev < kMaxDevices, "grouped_gemm: device index %d out of range", dev);
-  if (done[dev].load(std::memory_order_acquire)) return BOLT_OK;
-  cudaFuncAttributes attr;
-  BOLT_CUDA(cudaFuncGetAttributes(&attr, kfn));
-  if (dec_threads > 0 &&
-      (int64_t)dec_threads * (attr.numRegs - dec_regs) < (int64_t)inc_threads * (inc_regs - attr.numRegs)) {
-    set_error("grouped_gemm: kernel was built with %d registers per thread; the register split "
-              "%d x %d -> %d / %d x %d -> %d cannot balance, refusing to launch",
-              attr.numRegs, dec_threads, attr.numRegs, dec_regs, inc_threads, attr.numRegs, inc_regs);
-    return BOLT_ERR_UNSUPPORTED;
-  }
-  BOLT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-  done[dev].store(true, std::memory_order_release);
-  return BOLT_OK;
-}
-
 template <int OPK, bool BS, int EPI, bool PAIR>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc,
            const GemmParams& p, int grid, cudaStream_t st) {
@@ -1633,9 +1606,19 @@ extern "C" int bolt_grouped_gemm(const bolt_gemm_args* a, void* stream) {
   BOLT_REQUIRE(!a->mul_routed_weight || a->sorted_weights,
                "grouped_gemm: mul_routed_weight needs sorted_weights");
 
-  BOLT_REQUIRE(a->schedule == BOLT_GEMM_SCHEDULE_ROW_TILES ||
-                   a->schedule == BOLT_GEMM_SCHEDULE_TILE_PAIRS,
+  BOLT_REQUIRE(a->schedule >= BOLT_GEMM_SCHEDULE_ROW_TILES &&
+                   a->schedule <= BOLT_GEMM_SCHEDULE_STREAM,
                "grouped_gemm: unknown schedule %d", a->schedule);
+  const bool stream_weights = a->schedule == BOLT_GEMM_SCHEDULE_STREAM;
+  if (stream_weights) {
+    BOLT_REQUIRE(!mx && a->scatter_src == nullptr,
+                 "grouped_gemm: the streaming schedule is not built for the MX kind or "
+                 "segment-scattered output");
+    BOLT_REQUIRE(a->sorted_ids != nullptr && ((int64_t)a->k * elem) % 128 == 0,
+                 "grouped_gemm: the streaming schedule needs sorted_ids and k in whole 128-byte blocks");
+    BOLT_REQUIRE(!block || (a->a_scale_ld % 4 == 0 && reinterpret_cast<uintptr_t>(a->a_scale) % 16 == 0),
+                 "grouped_gemm: the streaming schedule needs 16-byte aligned activation scales");
+  }
   const bool pair = a->schedule == BOLT_GEMM_SCHEDULE_TILE_PAIRS;
   if (pair) {
     BOLT_REQUIRE(!mx, "grouped_gemm: the tile-pair schedule is not built for the MX kind");
@@ -1699,6 +1682,8 @@ extern "C" int bolt_grouped_gemm(const bolt_gemm_args* a, void* stream) {
       return BOLT_ERR_CUDA;
     }
   }
+
+  if (stream_weights) return stream_gemm(a, mb, st);
 
   GemmParams p{};
   p.a_scale = a->a_scale;

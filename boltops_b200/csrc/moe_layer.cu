@@ -107,6 +107,9 @@ int check_args(const bolt_layer_args* a) {
                  "moe_layer: hidden_states dtype does not match the weights");
   else
     BOLT_REQUIRE(a->w1_scale && a->w2_scale, "moe_layer: weight scales required");
+  BOLT_REQUIRE(a->schedule == BOLT_GEMM_SCHEDULE_ROW_TILES ||
+                   a->schedule == BOLT_GEMM_SCHEDULE_STREAM,
+               "moe_layer: schedule %d is not built into the one-call layer", a->schedule);
   if (block)
     BOLT_REQUIRE(a->hidden % 128 == 0 && a->inter % 128 == 0,
                  "moe_layer: block-scaled experts need hidden and intermediate sizes in 128s");
@@ -196,6 +199,7 @@ extern "C" int bolt_moe_layer(const bolt_layer_args* a, void* stream) {
   g.status = a->status;
   g.mid_dtype = a->out_dtype;
   g.bias_dtype = a->bias_dtype;
+  g.schedule = a->schedule;
 
   // ---- GEMM 1: gate / up with SiLU(gate) * up (and the 1x128 re-quantisation) in the epilogue
   void* a2 = ws + p.off_a2;

@@ -5,6 +5,8 @@
 
 #include <cuda.h>
 
+#include <atomic>
+
 #include "common.cuh"
 
 namespace bolt {
@@ -337,6 +339,34 @@ __device__ __forceinline__ void round2(float& a, float& b) {
   }
 }
 
+constexpr int kMaxDevices = 64;
+
+// One-time set-up of a kernel on the CURRENT device (`done` has one slot per device ordinal):
+// the dynamic shared-memory opt-in is a per-device attribute, and a kernel that re-splits its
+// registers with setmaxnreg must have been compiled to a register count from which the split
+// balances -- `setmaxnreg.inc` only gets registers that `setmaxnreg.dec` released in the same
+// CTA and waits forever otherwise, so an unbalanced split is refused here instead of launched.
+// dec_threads drop to dec_regs, inc_threads rise to inc_regs (0 threads: no split).
+template <typename KernelT>
+int configure_kernel(KernelT kfn, int smem_bytes, std::atomic<bool>* done, int dec_threads,
+                     int dec_regs, int inc_threads, int inc_regs) {
+  int dev = 0;
+  BOLT_CUDA(cudaGetDevice(&dev));
+  BOLT_REQUIRE(dev >= 0 && dev < kMaxDevices, "grouped_gemm: device index %d out of range", dev);
+  if (done[dev].load(std::memory_order_acquire)) return BOLT_OK;
+  cudaFuncAttributes attr;
+  BOLT_CUDA(cudaFuncGetAttributes(&attr, kfn));
+  if (dec_threads > 0 &&
+      (int64_t)dec_threads * (attr.numRegs - dec_regs) < (int64_t)inc_threads * (inc_regs - attr.numRegs)) {
+    set_error("grouped_gemm: kernel was built with %d registers per thread; the register split "
+              "%d x %d -> %d / %d x %d -> %d cannot balance, refusing to launch",
+              attr.numRegs, dec_threads, attr.numRegs, dec_regs, inc_threads, attr.numRegs, inc_regs);
+    return BOLT_ERR_UNSUPPORTED;
+  }
+  BOLT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
+  done[dev].store(true, std::memory_order_release);
+  return BOLT_OK;
+}
 
 }  // namespace tc
 }  // namespace bolt

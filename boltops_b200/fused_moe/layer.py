@@ -119,6 +119,28 @@ def _use_tile_pairs(kind: int, routes: int, experts: int) -> bool:
 _PAIR_MIN_AVG_ROWS = 384
 
 
+def _use_stream(kind: int, routes: int, experts: int, hidden: int, inter: int) -> bool:
+    """Whether the two GEMMs run in the weight-streaming form (``csrc/stream_gemm.cuh``), which
+    computes only live rows and is bound by HBM up to about 32 of them per expert.  Equal results, so
+    the line is one of speed alone, both sides measured in us per layer (row tiles / streaming).
+    Block-scaled kinds, whose promotion needs a scale per row there: DeepSeek-V3 fp8, 3 routes per
+    expert 1934 / 1877, 8: 2011 / 1985, 16: 2134 / 2121, 50: 308 / 337 (32 experts); Zipf-distributed
+    routing at 16 routes per expert (hot experts of 200) 482 / 472.  The others: Mixtral bf16, 16
+    routes per expert 482 / 461, Qwen3-30B int8, 32: 202 / 191, Mixtral 100: 475 / 621.
+    ``BOLTOPS_B200_GEMM_SCHEDULE`` = ``stream`` forces it, ``tiles`` / ``pairs`` rule it out."""
+    elem = 2 if kind in (_cabi.GEMM_BF16, _cabi.GEMM_F16) else 1
+    if (hidden * elem) % 128 or (inter * elem) % 128:
+        return False
+    forced = os.environ.get("BOLTOPS_B200_GEMM_SCHEDULE", "auto")
+    if forced != "auto":
+        return forced == "stream"
+    block = kind in (_cabi.GEMM_FP8_BLOCK, _cabi.GEMM_INT8_BLOCK)
+    return routes <= (_STREAM_MAX_AVG_ROWS_BLOCK if block else _STREAM_MAX_AVG_ROWS) * experts
+
+
+_STREAM_MAX_AVG_ROWS, _STREAM_MAX_AVG_ROWS_BLOCK = 32, 16
+
+
 def gemm_schedule(kind: int, routes: int, experts: int) -> str:
     """Name of the schedule ``fused_experts`` picks for this problem ("pairs" / "tiles")."""
     return "pairs" if _use_tile_pairs(kind, routes, experts) else "tiles"
@@ -360,6 +382,8 @@ def fused_experts_impl(
         args.routed_scaling_factor = float(routed_scaling_factor)
         args.out = out.data_ptr()
         args.status = ops.device_status(dev).data_ptr()
+        if _use_stream(kind, num_tokens * topk, global_num_experts, hidden, act_dim):
+            args.schedule = _cabi.SCHEDULE_STREAM
         lib = _cabi.load()
         need = lib.bolt_moe_layer_workspace_bytes(args)
         if need == 0:
@@ -435,7 +459,9 @@ def fused_experts_impl(
 
         common = dict(kind=kind, sorted_expert_ids=expert_ids, num_valid=num_valid,
                       sorted_ids=sorted_ids, sorted_weights=sorted_w, num_tokens=m, topk=topk,
-                      segments=segments, num_segments=num_segments)
+                      segments=segments, num_segments=num_segments,
+                      stream=segments is None and _out_peers is None
+                      and _use_stream(kind, m * topk, global_num_experts, hidden, act_dim))
 
         # ---- GEMM1 (+ activation, + re-quantisation) ---------------------------------------
         act_scale = None

@@ -536,12 +536,14 @@ def grouped_gemm(*, kind: int, epilogue: int, a: torch.Tensor, b: torch.Tensor, 
                  act_limit: Optional[float] = None, segments: Optional[torch.Tensor] = None,
                  num_segments: Optional[torch.Tensor] = None,
                  a_gather: bool = False, scatter_src: Optional[torch.Tensor] = None,
-                 scatter_seg_off: Optional[torch.Tensor] = None, scatter_seg_rows: int = 0) -> None:
+                 scatter_seg_off: Optional[torch.Tensor] = None, scatter_seg_rows: int = 0,
+                 stream: bool = False) -> None:
     """One grouped expert GEMM launch (see ``bolt_grouped_gemm``).  With ``segments`` (from
     ``moe_sorting_ck(..., segment_rows=PAIR_SEGMENT_ROWS)``) the tile-pair schedule runs.  With
     ``a_gather`` the row operand ``a`` is in TOKEN order and the kernel gathers its rows through
     ``sorted_ids`` (padding positions read zeros).  ``scatter_src`` / ``scatter_seg_off`` /
-    ``scatter_seg_rows``: scattered rows go to per-segment regions (see ``bolt_gemm_args``)."""
+    ``scatter_seg_rows``: scattered rows go to per-segment regions (see ``bolt_gemm_args``).
+    ``stream`` selects the weight-streaming schedule (experts with a handful of rows)."""
     lib = _cabi.load()
     args = _cabi.GemmArgs()
     args.kind = kind
@@ -592,6 +594,8 @@ def grouped_gemm(*, kind: int, epilogue: int, a: torch.Tensor, b: torch.Tensor, 
         args.scatter_src = ptr(scatter_src)
         args.scatter_seg_off = ptr(scatter_seg_off)
         args.scatter_seg_rows = scatter_seg_rows
+    if stream:
+        args.schedule = _cabi.SCHEDULE_STREAM
     if segments is not None:
         args.schedule = _cabi.SCHEDULE_TILE_PAIRS
         args.max_segments = segments.shape[0]

@@ -78,11 +78,16 @@ enum bolt_gemm_kind {
 /* grouped-GEMM schedules */
 enum bolt_gemm_schedule {
   BOLT_GEMM_SCHEDULE_ROW_TILES = 0,  /* one CTA per 128-row x 256-column tile                      */
-  BOLT_GEMM_SCHEDULE_TILE_PAIRS = 1  /* two CTAs of a cluster share the weight tile of two row
+  BOLT_GEMM_SCHEDULE_TILE_PAIRS = 1, /* two CTAs of a cluster share the weight tile of two row
                                         tiles of one expert (tcgen05 cta_group::2, 256 x 256 per
                                         pair): for experts with several row tiles.  Needs the
                                         segment list of bolt_moe_sort_ck with segment_rows =
                                         BOLT_PAIR_SEGMENT_ROWS; not for the MX kind.               */
+  BOLT_GEMM_SCHEDULE_STREAM = 2      /* weights streamed through small matrix instructions, only the
+                                        live rows of a tile computed: for experts with a handful of
+                                        rows.  Needs sorted_ids and k in whole 128-byte blocks; rows
+                                        that pad a tile are not written; not for the MX kind, no
+                                        segment-scattered output.                                  */
 };
 #define BOLT_PAIR_SEGMENT_ROWS 256
 
@@ -553,6 +558,7 @@ typedef struct bolt_layer_args {
   void* workspace;
   size_t workspace_bytes;
   int32_t* status;             /* optional, as in bolt_gemm_args                              */
+  int schedule;                /* enum bolt_gemm_schedule of both GEMMs: ROW_TILES or STREAM    */
 } bolt_layer_args;
 
 /* kernels one bolt_moe_layer call with these arguments launches (-1: invalid arguments) */

@@ -62,6 +62,7 @@ class GemmArgs(C.Structure):
         ("segments", C.c_void_p), ("num_segments", C.c_void_p),
         ("a_gather", C.c_int), ("a_rows", C.c_int), ("a_row_bytes", C.c_int64),
         ("scatter_src", C.c_void_p), ("scatter_seg_off", C.c_void_p), ("scatter_seg_rows", C.c_int),
+        ("a_scale_token_order", C.c_int),
     ]
 
 

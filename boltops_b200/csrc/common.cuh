@@ -96,6 +96,10 @@ __device__ __forceinline__ int8_t f32_to_i8(float v) {
   return (int8_t)(int)r;
 }
 
+// bolt_quant_rows; with rows_dev (device memory) rows past that count may be left as they are.
+int quant_rows(const void* x, int x_dtype, int64_t rows, int cols, int group, int q_dtype, int power2,
+               void* q, float* scales, int64_t scales_ld, const int32_t* rows_dev, cudaStream_t st);
+
 // 16-byte vector of N elements of T.
 template <typename T, int N>
 struct alignas(sizeof(T) * N) Vec {

@@ -115,6 +115,7 @@ struct GemmParams {
   // gathered row operand: A is in TOKEN order; sorted position p reads row (sorted_ids[p] & 0xFFFFFF),
   // or zeros when that id is not a token (tile padding)
   int a_gather;
+  int a_scale_tok;   // channel kinds: a_scale is indexed by token
   const void* a_base;
   int a_row_units;   // 16-byte units between rows
   int k_bytes;
@@ -754,7 +755,11 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       const int r = c.m_blk * kBM + row_in_tile;
       m.sid = has_ids ? p.sorted_ids[r] : 0;
       m.rw = has_rw ? p.sorted_weights[r] : 1.0f;
-      m.a_s = CHANNEL ? p.a_scale[r] : 1.0f;
+      m.a_s = 1.0f;
+      if (CHANNEL) {
+        const int token = m.sid & 0xFFFFFF;
+        m.a_s = p.a_scale[p.a_scale_tok ? (token < p.num_tokens ? token : 0) : r];
+      }
       m.col_s = 1.0f;
       m.col_b = 0.0f;
       if (!BS && (CHANNEL || p.bias != nullptr) && m.expert >= 0 && m.expert < p.num_experts) {
@@ -1627,6 +1632,9 @@ extern "C" int bolt_grouped_gemm(const bolt_gemm_args* a, void* stream) {
   }
 
   const bool gather = a->a_gather != 0;
+  BOLT_REQUIRE(!a->a_scale_token_order ||
+                   (gather && (a->kind == BOLT_GEMM_FP8_CHANNEL || a->kind == BOLT_GEMM_INT8_CHANNEL)),
+               "grouped_gemm: row scales in token order go with gathered rows of the per-channel kinds");
   if (gather) {
     BOLT_REQUIRE(!pair && !mx, "grouped_gemm: the gathered row operand needs the single-tile "
                                "schedule of the plain kinds");
@@ -1750,6 +1758,7 @@ extern "C" int bolt_grouped_gemm(const bolt_gemm_args* a, void* stream) {
     if (pair) p.group_m = (p.group_m + 1) / 2;   // the unit of the tile order is a pair of row tiles
   }
   p.a_gather = gather ? 1 : 0;
+  p.a_scale_tok = a->a_scale_token_order;
   p.a_base = a->a;
   p.a_row_units = (int)((a->a_row_bytes > 0 ? a->a_row_bytes : (int64_t)a->k * elem) / 16);
   p.k_bytes = a->k * elem;

@@ -27,7 +27,10 @@ constexpr int kUnit = 128;
 // sorted layout is mostly tile padding (measured on the DeepSeek-V3 fp8 layer: 0.120 vs 0.152 ms
 // at 8 routes, 0.49 vs 0.52 ms at 16 routes per expert, even at 128, 4.56 vs 4.51 ms at 256
 // routes per expert, where the extra copy instructions slow the accumulator promotion down), so
-// it is used up to kGatherMaxAvgRows routes per expert.  BOLTOPS_B200_GATHER=0 / 1 forces it off
+// it is used up to kGatherMaxAvgRows routes per expert.  The per-channel kinds have no promotion to
+// slow down, and their rows in token order stay in L2 where the sorted copy does not: there it is
+// used from that size on (Qwen3-30B int8: 16384 tokens, sorted copy + GEMM 1 93 + 363 us, gathered
+// 400 us; 1200 tokens 10 + 87 against 82 us).  BOLTOPS_B200_GATHER=0 / 1 forces it off
 // / on.
 constexpr int kGatherMaxAvgRows = 64;
 bool gather_rows_in_gemm(const bolt_layer_args* a) {
@@ -37,7 +40,8 @@ bool gather_rows_in_gemm(const bolt_layer_args* a) {
     return std::strcmp(v, "0") != 0 ? 1 : 0;
   }();
   if (forced >= 0) return forced == 1;
-  return (int64_t)a->num_tokens * a->topk <= (int64_t)kGatherMaxAvgRows * a->global_num_experts;
+  const bool few = (int64_t)a->num_tokens * a->topk <= (int64_t)kGatherMaxAvgRows * a->global_num_experts;
+  return a->kind == BOLT_GEMM_INT8_CHANNEL || a->kind == BOLT_GEMM_FP8_CHANNEL ? !few : few;
 }
 
 inline size_t a256(size_t n) { return (n + 255) & ~size_t(255); }
@@ -63,7 +67,7 @@ int make_plan(const bolt_layer_args* a, Plan& p) {
   p.block = a->kind == BOLT_GEMM_FP8_BLOCK || a->kind == BOLT_GEMM_INT8_BLOCK;
   p.quant = !p.is16;
   p.qbytes = p.is16 ? 2 : 1;
-  p.gather = (p.block || p.is16) && gather_rows_in_gemm(a);
+  p.gather = gather_rows_in_gemm(a);
   const int osz = dtype_bytes(a->out_dtype);
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o += a256(bytes); return at; };
@@ -75,10 +79,11 @@ int make_plan(const bolt_layer_args* a, Plan& p) {
   p.off_route_pos = take((size_t)routes * 4);
   p.sort_ws_bytes = bolt_moe_sort_workspace_bytes(a->num_tokens, a->topk, a->global_num_experts);
   p.off_sort_ws = take(p.sort_ws_bytes);
-  p.off_a1 = take(p.gather ? (p.is16 ? 0 : (size_t)a->num_tokens * a->hidden)
+  p.off_a1 = take(p.gather ? (p.block ? (size_t)a->num_tokens * a->hidden : 0)
                            : (size_t)p.cap * a->hidden * p.qbytes);
-  p.off_a1_scale = take(p.block ? (size_t)(a->hidden / 128) * p.cap * 4 : (p.quant ? (size_t)p.cap * 4 : 0));
-  // per-channel kinds quantise every token once, then gather codes and scales
+  p.off_a1_scale = take(p.block ? (size_t)(a->hidden / 128) * p.cap * 4
+                                : (p.quant && !p.gather ? (size_t)p.cap * 4 : 0));
+  // per-channel kinds quantise every token once; GEMM 1 gathers codes and scales, or a pass before it
   p.off_xq = take(p.quant && !p.block ? (size_t)a->num_tokens * a->hidden : 0);
   p.off_xq_scale = take(p.quant && !p.block ? (size_t)a->num_tokens * 4 : 0);
   p.off_a2 = take((size_t)p.cap * a->inter * p.qbytes);
@@ -132,7 +137,7 @@ extern "C" int bolt_moe_layer_kernel_count(const bolt_layer_args* a) {
   if (check_args(a) != BOLT_OK || make_plan(a, p) != BOLT_OK) return -1;
   if (a->num_tokens == 0) return 0;
   const int sort = p.sort_ws_bytes <= 16 ? 1 : 2;
-  const int place = p.block ? 1 : (p.quant ? 2 : (p.gather ? 0 : 1));
+  const int place = p.block ? 1 : (p.gather ? 0 : 1) + (p.quant ? 1 : 0);
   return sort + place + 2 + (p.quant && !p.block ? 1 : 0) + 1;
 }
 
@@ -177,7 +182,7 @@ extern "C" int bolt_moe_layer(const bolt_layer_args* a, void* stream) {
   } else if (p.quant) {
     rc = bolt_quant_rows(a->hidden_states, a->x_dtype, a->num_tokens, a->hidden, a->hidden,
                          q_dtype, 0, ws + p.off_xq, f32(p.off_xq_scale), 0, stream);
-    if (rc == BOLT_OK)
+    if (rc == BOLT_OK && !p.gather)
       rc = bolt_gather_rows(ws + p.off_xq, a->num_tokens, a->hidden, 0, f32(p.off_xq_scale), 0, 1,
                             sorted_ids, num_valid, p.cap, a1, a1_scale, p.cap, stream);
   } else if (!p.gather) {
@@ -206,10 +211,11 @@ extern "C" int bolt_moe_layer(const bolt_layer_args* a, void* stream) {
   float* a2_scale = p.quant ? f32(p.off_a2_scale) : nullptr;
   g.n = 2 * a->inter;
   g.k = a->hidden;
-  g.a = (p.gather && p.is16) ? a->hidden_states : a1;
+  g.a = !p.gather || p.block ? a1 : p.is16 ? a->hidden_states : ws + p.off_xq;
   g.b = a->w1;
-  g.a_scale = a1_scale;
+  g.a_scale = p.gather && p.quant && !p.block ? f32(p.off_xq_scale) : a1_scale;
   g.a_scale_ld = p.cap;
+  g.a_scale_token_order = p.gather && p.quant && !p.block;
   g.b_scale = a->w1_scale;
   g.bias = a->b1;
   g.mul_routed_weight = a->apply_router_weight_on_input;
@@ -233,13 +239,14 @@ extern "C" int bolt_moe_layer(const bolt_layer_args* a, void* stream) {
   rc = bolt_grouped_gemm(&g, stream);
   if (rc != BOLT_OK) return rc;
   if (p.quant && !p.block) {
-    rc = bolt_quant_rows(ws + p.off_actf, a->out_dtype, p.cap, a->inter, a->inter, q_dtype, 0, a2,
-                         a2_scale, 0, stream);
+    rc = quant_rows(ws + p.off_actf, a->out_dtype, p.cap, a->inter, a->inter, q_dtype, 0, a2, a2_scale,
+                    0, num_valid, static_cast<cudaStream_t>(stream));
     if (rc != BOLT_OK) return rc;
   }
 
   // ---- GEMM 2: down projection, router weight in the epilogue, rows stay in sorted order
   g.a_gather = 0;
+  g.a_scale_token_order = 0;
   g.epilogue = BOLT_EPI_STORE;
   g.n = a->model_dim;
   g.k = a->inter;

@@ -30,6 +30,7 @@ int stream_gemm(const bolt_gemm_args* a, const CUtensorMap& mb, cudaStream_t st)
   p.c_scale = a->c_scale;
   p.c_scale_ld = a->c_scale_ld;
   p.gather = a->a_gather != 0;
+  p.a_scale_tok = a->a_scale_token_order;
   p.scatter = a->scatter;
   p.num_tokens = a->num_tokens;
   p.topk = a->topk;

@@ -72,7 +72,7 @@ struct StreamParams {
   int64_t c_ld;
   float* c_scale;
   int64_t c_scale_ld;
-  int gather, scatter, num_tokens, topk, mul_routed_weight, c_vec_ok;
+  int gather, a_scale_tok, scatter, num_tokens, topk, mul_routed_weight, c_vec_ok;
   const int32_t* sorted_ids;
   const float* sorted_weights;
   const int32_t* expert_ids;
@@ -309,7 +309,8 @@ __device__ __forceinline__ bool finish_item(const StreamParams& p, Epilogue& ep,
       const int r = (u >> 3) * t_cols + 8 * k + (u & 7);
       if (r >= rows) continue;                   // warp-uniform
       const int row = row0 + r;
-      const float a_s = CHANNEL ? __ldg(p.a_scale + row) : 1.f;
+      const float a_s =
+          CHANNEL ? __ldg(p.a_scale + (p.a_scale_tok ? p.sorted_ids[row] & 0xFFFFFF : row)) : 1.f;
       const float rw = has_rw ? __ldg(p.sorted_weights + row) : 1.f;
       float y[G][V];
 #pragma unroll

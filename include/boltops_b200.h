@@ -517,6 +517,8 @@ typedef struct bolt_gemm_args {
   const int32_t* scatter_src;
   const int64_t* scatter_seg_off;
   int scatter_seg_rows;
+  int a_scale_token_order; /* per-channel kinds with a_gather: a_scale is indexed by token, not by
+                              sorted position                                                */
 } bolt_gemm_args;
 
 int bolt_grouped_gemm(const bolt_gemm_args* args, void* stream);

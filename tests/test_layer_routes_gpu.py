@@ -1,0 +1,32 @@
+"""Routes through the layer that depend on sizes, against the routes they replace."""
+import pytest
+import torch
+
+from oracle import moe_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m", [257, 300])        # just above 64 routes per expert / more than a tile
+@pytest.mark.parametrize("hidden", [512, 2064])  # 2064: a reduction tail of 16 bytes
+@pytest.mark.parametrize("bias", [False, True])
+def test_per_channel_rows_gathered_by_the_gemm(monkeypatch, m, hidden, bias):
+    """From 64 routes per expert on GEMM 1 of the per-channel kinds reads codes and scales in token
+    order; the kernel-by-kernel orchestration still places sorted rows.  Equal bit for bit."""
+    from boltops_b200.fused_moe import fused_experts, layer
+    e, topk, inter = 8, 2, 256
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn(m, hidden, generator=g).bfloat16().cuda()
+    w1, s1 = O.quantize_weight_channel_int8(torch.randn(e, 2 * inter, hidden, generator=g) * 0.05)
+    w2, s2 = O.quantize_weight_channel_int8(torch.randn(e, hidden, inter, generator=g) * 0.05)
+    wts, ids = O.make_routing(m, e, topk, 9)
+    ids[3, 1] = -1
+    kw = dict(use_int8_w8a8=True, per_channel_quant=True, w1_scale=s1.cuda(), w2_scale=s2.cuda())
+    if bias:
+        kw.update(b1=torch.randn(e, 2 * inter, generator=g).bfloat16().cuda(),
+                  b2=torch.randn(e, hidden, generator=g).bfloat16().cuda())
+    args = (x, w1.cuda(), w2.cuda(), wts.cuda(), ids.cuda())
+    one = fused_experts(*args, **kw)
+    monkeypatch.setattr(layer, "_ONE_CALL", False)
+    steps = fused_experts(*args, **kw)
+    assert torch.equal(one.cpu(), steps.cpu())

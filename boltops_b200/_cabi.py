@@ -62,7 +62,7 @@ class GemmArgs(C.Structure):
         ("segments", C.c_void_p), ("num_segments", C.c_void_p),
         ("a_gather", C.c_int), ("a_rows", C.c_int), ("a_row_bytes", C.c_int64),
         ("scatter_src", C.c_void_p), ("scatter_seg_off", C.c_void_p), ("scatter_seg_rows", C.c_int),
-        ("a_scale_token_order", C.c_int),
+        ("a_scale_token_order", C.c_int), ("dense_rows", C.c_int),
     ]
 
 
@@ -111,6 +111,8 @@ _SIGNATURES = {
                                     C.c_void_p, C.c_int64, C.c_void_p]),
     "bolt_quant_rows": (C.c_int, [C.c_void_p, C.c_int, C.c_int64, C.c_int, C.c_int, C.c_int,
                                   C.c_int, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]),
+    "bolt_dense_prep": (C.c_int, [C.c_void_p, C.c_int64, C.c_int, C.c_void_p, C.c_int64, C.c_void_p,
+                                  C.c_void_p, C.c_void_p]),
     "bolt_quant_scatter_rows": (C.c_int, [C.c_void_p, C.c_int, C.c_int64, C.c_int, C.c_int, C.c_int,
                                           C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p,
                                           C.c_int, C.c_void_p, C.c_void_p, C.c_int64, C.c_int,

@@ -101,6 +101,7 @@ struct GemmParams {
   int k;
   int num_experts;
   int capacity;
+  int rows;          // rows that exist in a and c (dense operands; else the capacity)
   int tiles_n;
   int num_kb;
   int kb_scale_cols;  // k/128 (block-scaled kinds)
@@ -820,7 +821,7 @@ k_grouped_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       const int row = tc.m_blk * kBM + row_in_tile;
       const int tile_row0 = tc.m_blk * kBM + 32 * q;   // output row of lane 0 (sorted layout)
       const int token = cur.sid & 0xFFFFFF;
-      const bool live = token < p.num_tokens && cur.has_tile;
+      const bool live = token < p.num_tokens && cur.has_tile && row < p.rows;
       // Gated epilogues feed the next GEMM: padding rows are written as zeros rather than left
       // as stale memory, because operand rows full of arbitrary bits cost tensor-core power
       // (and with it SM clock) in the GEMM that streams them.
@@ -1632,6 +1633,11 @@ extern "C" int bolt_grouped_gemm(const bolt_gemm_args* a, void* stream) {
   }
 
   const bool gather = a->a_gather != 0;
+  BOLT_REQUIRE(a->dense_rows == 0 ||
+                   (a->dense_rows > 0 && a->dense_rows <= a->capacity && a->sorted_ids == nullptr &&
+                    a->schedule == BOLT_GEMM_SCHEDULE_ROW_TILES && !mx && a->epilogue == BOLT_EPI_STORE),
+               "grouped_gemm: dense_rows is for row tiles without sorted_ids and a plain epilogue");
+  const int rows = a->dense_rows > 0 ? a->dense_rows : a->capacity;   // that exist in a and c
   BOLT_REQUIRE(!a->a_scale_token_order ||
                    (gather && (a->kind == BOLT_GEMM_FP8_CHANNEL || a->kind == BOLT_GEMM_INT8_CHANNEL)),
                "grouped_gemm: row scales in token order go with gathered rows of the per-channel kinds");
@@ -1660,7 +1666,8 @@ extern "C" int bolt_grouped_gemm(const bolt_gemm_args* a, void* stream) {
   CUtensorMap ma, mb;
   {
     // (with a gathered row operand this map is not used by the kernel)
-    cuuint64_t dims[2] = {(cuuint64_t)a->k, (cuuint64_t)(gather ? a->a_rows : a->capacity)};
+    // (rows past the end of a dense operand read as zeros)
+    cuuint64_t dims[2] = {(cuuint64_t)a->k, (cuuint64_t)(gather ? a->a_rows : rows)};
     cuuint64_t strides[1] = {gather && a->a_row_bytes > 0 ? (cuuint64_t)a->a_row_bytes
                                                           : (cuuint64_t)a->k * elem};
     cuuint32_t box[2] = {bk, (cuuint32_t)kBM};
@@ -1720,7 +1727,8 @@ extern "C" int bolt_grouped_gemm(const bolt_gemm_args* a, void* stream) {
   if (p.c_vec_ok && !a->scatter && (out8 || a->c_dtype == BOLT_BF16 || a->c_dtype == BOLT_F16)) {
     const int64_t out_cols = gated ? a->n / 2 : a->n;
     const int esz = out8 ? 1 : 2;
-    cuuint64_t dims[2] = {(cuuint64_t)out_cols, (cuuint64_t)a->capacity};
+    cuuint64_t dims[2] = {(cuuint64_t)out_cols,
+                          (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)a->c_ld * esz};
     cuuint32_t box[2] = {(cuuint32_t)(64 / esz), 32};   // 64 bytes x 32 rows either way
     cuuint32_t estr[2] = {1, 1};
@@ -1743,6 +1751,7 @@ extern "C" int bolt_grouped_gemm(const bolt_gemm_args* a, void* stream) {
   p.k = a->k;
   p.num_experts = a->num_experts;
   p.capacity = a->capacity;
+  p.rows = rows;
   p.tiles_n = gated ? (p.n_half + 127) / 128 : (a->n + 255) / 256;
   p.num_kb = (a->k + (int)bk - 1) / (int)bk;
   p.kb_scale_cols = a->k / 128;

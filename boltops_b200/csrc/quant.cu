@@ -329,6 +329,32 @@ int dispatch_quant(const void* x, int64_t rows, int cols, int group, int q_dtype
   return launch_quant<TIn, BOLT_INT8, false>(x, rows, cols, group, q, scales, rows_dev, st);
 }
 
+// ---- dense operands of the grouped GEMM -------------------------------------------
+// Row-major activation scales [rows, groups] -> group-major [groups, ld], zeros past the last row,
+// plus what a grouped GEMM over one "expert" reads: tile labels (all 0) and the number of rows.
+// A 32 x 32 tile per block, both sides coalesced.
+__global__ void __launch_bounds__(256) k_dense_prep(const float* __restrict__ src, int64_t rows,
+                                                    int groups, float* __restrict__ dst, int64_t ld,
+                                                    int32_t* __restrict__ tile_ids, int tiles,
+                                                    int32_t* __restrict__ num_rows) {
+  __shared__ float t[32][33];
+  const int64_t r0 = (int64_t)blockIdx.x * 32;
+  const int g0 = blockIdx.y * 32;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < 32; i += 8)
+    t[y + i][x] = (r0 + y + i < rows && g0 + x < groups) ? src[(r0 + y + i) * groups + g0 + x] : 0.f;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 32; i += 8)
+    if (g0 + y + i < groups) dst[(int64_t)(g0 + y + i) * ld + r0 + x] = t[x][y + i];
+  if (blockIdx.y == 0) {
+    const int tid = blockIdx.x * 256 + threadIdx.x;
+    if (tid < tiles) tile_ids[tid] = 0;
+    if (tid == 0) *num_rows = (int32_t)ld;
+  }
+}
+
 // ---- gather into expert-sorted rows ----------------------------------------------
 __global__ void __launch_bounds__(256) k_gather_rows(const uint4* __restrict__ src,
                                                      int num_tokens, int row_vecs,
@@ -777,6 +803,21 @@ extern "C" int bolt_quant_rows(const void* x, int x_dtype, int64_t rows, int col
                                int64_t scales_ld, void* stream) {
   return bolt::quant_rows(x, x_dtype, rows, cols, group, q_dtype, power2, q, scales_ptr, scales_ld,
                           nullptr, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int bolt_dense_prep(const float* a_scale, int64_t rows, int groups, float* a_scale_t,
+                               int64_t ld, int32_t* tile_ids, int32_t* num_rows, void* stream) {
+  using namespace bolt;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  BOLT_REQUIRE(rows > 0 && groups > 0 && ld >= rows && ld % 128 == 0 && ld < (1ll << 30),
+               "dense_prep: bad shape");
+  BOLT_REQUIRE(groups <= 32 * 65535, "dense_prep: too many groups");
+  BOLT_REQUIRE(a_scale && a_scale_t && tile_ids && num_rows, "dense_prep: null pointer");
+  const dim3 grid((unsigned)(ld / 32), (unsigned)((groups + 31) / 32));
+  k_dense_prep<<<grid, 256, 0, st>>>(a_scale, rows, groups, a_scale_t, ld, tile_ids, (int)(ld / 128),
+                                     num_rows);
+  BOLT_LAUNCH_CHECK();
+  return BOLT_OK;
 }
 
 extern "C" int bolt_gather_rows(const void* src, int num_tokens, int row_bytes,

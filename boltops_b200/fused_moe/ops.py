@@ -523,6 +523,14 @@ def check_device_status(device: torch.device) -> None:
                               f"GEMM, 20 exchange barrier, 21 exchange segment overflow)")
 
 
+def gemm_sm_count(device) -> int:
+    """SMs a grouped GEMM may use on ``device`` (0: all of them)."""
+    if _gemm_sm_reserve <= 0:
+        return 0
+    total = torch.cuda.get_device_properties(device).multi_processor_count
+    return max(total - _gemm_sm_reserve, 1)
+
+
 def grouped_gemm(*, kind: int, epilogue: int, a: torch.Tensor, b: torch.Tensor, c: torch.Tensor,
                  sorted_expert_ids: torch.Tensor, num_valid: torch.Tensor,
                  a_scale: Optional[torch.Tensor] = None, a_scale_ld: int = 0,
@@ -581,10 +589,7 @@ def grouped_gemm(*, kind: int, epilogue: int, a: torch.Tensor, b: torch.Tensor, 
     args.sorted_expert_ids = ptr(sorted_expert_ids)
     args.num_valid_ids = ptr(num_valid)
     args.status = ptr(device_status(a.device))
-    if sm_count == 0 and _gemm_sm_reserve > 0:
-        total = torch.cuda.get_device_properties(a.device).multi_processor_count
-        sm_count = max(total - _gemm_sm_reserve, 1)
-    args.sm_count = sm_count
+    args.sm_count = sm_count or gemm_sm_count(a.device)
     args.act_alpha = float(act_alpha)
     args.act_beta = float(act_beta)
     args.act_limit = float(act_limit or 0.0)

@@ -38,29 +38,41 @@ def gemm_a8w8_blockscale(x: torch.Tensor, w: torch.Tensor, x_scale: torch.Tensor
         raise ValueError("scale shapes do not match the 1x128 / 128x128 recipe")
     kind = _cabi.GEMM_FP8_BLOCK if x.dtype == torch.float8_e4m3fn else _cabi.GEMM_INT8_BLOCK
     dev = x.device
-    cap = ops.ceil_to(max(m, 1), 128)
-    x = x.contiguous()
-    if cap != m:
-        xp = torch.zeros((cap, k), dtype=x.dtype, device=dev)
-        xp[:m] = x
-        x = xp
-    a_scale = torch.zeros((k // 128, cap), dtype=torch.float32, device=dev)
-    a_scale[:, :m] = x_scale.float().t()
-    direct = out is not None and cap == m
     if out is not None:
         assert out.shape == (m, n) and out.dtype == dtype and out.is_contiguous()
-    c = out if direct else torch.empty((cap, n), dtype=dtype, device=dev)
-    expert_ids = torch.zeros(cap // 128, dtype=torch.int32, device=dev)
-    num_valid = torch.full((1,), cap, dtype=torch.int32, device=dev)
-    ops.grouped_gemm(kind=kind, epilogue=_cabi.EPI_STORE, a=x, b=w.contiguous().unsqueeze(0), c=c,
-                     sorted_expert_ids=expert_ids, num_valid=num_valid, a_scale=a_scale,
-                     a_scale_ld=cap, b_scale=w_scale.float().contiguous().unsqueeze(0))
-    if direct:
-        return out
-    if out is not None:
-        out.copy_(c[:m])
-        return out
-    return c[:m]
+    c = out if out is not None else torch.empty((m, n), dtype=dtype, device=dev)
+    if m == 0:
+        return c
+    # Two launches: the scales to group-major order (with the one "expert"'s tile labels), the GEMM.
+    # Rows that only pad the last row tile exist nowhere: the tensor map reads them as zeros and
+    # nothing is stored for them.
+    x, w = x.contiguous(), w.contiguous()
+    x_scale, w_scale = x_scale.float().contiguous(), w_scale.float().contiguous()
+    cap = ops.ceil_to(m, 128)
+    groups, tiles = k // 128, cap // 128
+    ws = torch.empty(groups * cap + tiles + 1, dtype=torch.float32, device=dev)
+    scale_t = ws.data_ptr()
+    tile_ids = scale_t + 4 * groups * cap
+    num_rows = tile_ids + 4 * tiles
+    args = _cabi.GemmArgs()
+    args.kind, args.epilogue = kind, _cabi.EPI_STORE
+    args.capacity, args.n, args.k, args.num_experts = cap, n, k, 1
+    args.a, args.b, args.c = x.data_ptr(), w.data_ptr(), c.data_ptr()
+    args.dense_rows = m
+    args.a_scale, args.a_scale_ld, args.b_scale = scale_t, cap, w_scale.data_ptr()
+    args.c_dtype = args.mid_dtype = _cabi.dtype_code(dtype)
+    args.c_ld, args.topk = n, 1
+    args.sorted_expert_ids, args.num_valid_ids = tile_ids, num_rows
+    args.status = ops.device_status(dev).data_ptr()
+    args.sm_count = ops.gemm_sm_count(dev)
+    lib = _cabi.load()
+    stream = _cabi.stream_of(x)
+    with _cabi.on_device(dev):
+        _cabi.check(lib.bolt_dense_prep(x_scale.data_ptr(), m, groups, scale_t, cap, tile_ids,
+                                        num_rows, stream))
+        _cabi.check(lib.bolt_grouped_gemm(args, stream))
+    ops._count(2)
+    return c
 
 
 def w8a8_block_scaled_mm(A: torch.Tensor, B: torch.Tensor, As: torch.Tensor, Bs: torch.Tensor,

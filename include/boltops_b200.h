@@ -248,6 +248,12 @@ int bolt_quant_rows(const void* x, int x_dtype, int64_t rows, int cols, int grou
                     int q_dtype, int power2, void* q, float* scales, int64_t scales_ld,
                     void* stream);
 
+/* Operands of a dense GEMM for bolt_grouped_gemm with one "expert": activation scales [rows, groups]
+ * -> [groups, ld] (ld = rows rounded up to 128; zeros past the last row), tile_ids [ld / 128] = 0,
+ * num_rows[0] = ld. */
+int bolt_dense_prep(const float* a_scale, int64_t rows, int groups, float* a_scale_t, int64_t ld,
+                    int32_t* tile_ids, int32_t* num_rows, void* stream);
+
 /* Row gather into the expert-sorted padded layout used by the grouped GEMMs.
  *   dst[i, :] = src[sorted_ids[i] & 0xFFFFFF, :] for i < num_valid_ids[0]
  *   (zero rows for pad ids); row_bytes must be a multiple of 16.
@@ -519,6 +525,8 @@ typedef struct bolt_gemm_args {
   int scatter_seg_rows;
   int a_scale_token_order; /* per-channel kinds with a_gather: a_scale is indexed by token, not by
                               sorted position                                                */
+  int dense_rows;          /* > 0: no sorted_ids, and only this many of the capacity's rows exist in `a`
+                              and `c` (plain epilogue, row-tile schedule)                    */
 } bolt_gemm_args;
 
 int bolt_grouped_gemm(const bolt_gemm_args* args, void* stream);

@@ -30,3 +30,25 @@ def test_per_channel_rows_gathered_by_the_gemm(monkeypatch, m, hidden, bias):
     monkeypatch.setattr(layer, "_ONE_CALL", False)
     steps = fused_experts(*args, **kw)
     assert torch.equal(one.cpu(), steps.cpu())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m", [1, 31, 127, 128, 129, 300])
+@pytest.mark.parametrize("n,k", [(128, 128), (384, 4224)])    # 4224: 33 scale groups
+def test_dense_rows_end_inside_a_tile(dtype, m, n, k):
+    """The dense GEMM reads no row past the last and writes none: the result of M rows equals the
+    first M rows of the result of a whole number of tiles, bit for bit, and lies in a guarded buffer."""
+    from boltops_b200.gemm import gemm_a8w8_blockscale
+    g = torch.Generator().manual_seed(m)
+    full = (m + 127) // 128 * 128
+    x = (torch.randn(full, k, generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn).cuda()
+    w = (torch.randn(n, k, generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn).cuda()
+    xs = (torch.rand(full, k // 128, generator=g) + 0.5).cuda()
+    ws = (torch.rand(n // 128, k // 128, generator=g) + 0.5).cuda()
+    whole = gemm_a8w8_blockscale(x, w, xs, ws, dtype=dtype)
+    buf = torch.full((full + 64, n), -7.0, dtype=dtype, device="cuda")
+    out = gemm_a8w8_blockscale(x[:m], w, xs[:m], ws, dtype=dtype, out=buf[:m])
+    assert torch.equal(out.cpu(), whole[:m].cpu())
+    assert (buf[m:] == -7.0).all()
+    some = gemm_a8w8_blockscale(x[:m], w, xs[:m].double(), ws, dtype=dtype)   # any floating scale type
+    assert torch.equal(some.cpu(), out.cpu())

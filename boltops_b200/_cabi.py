@@ -211,8 +211,9 @@ def ptr(t) -> int | None:
 
 
 def stream_of(t: torch.Tensor) -> int:
-    """Raw handle of torch's current stream on the tensor's device."""
-    return torch.cuda.current_stream(t.device).cuda_stream
+    """Raw handle of torch's current stream on the tensor's device (without the stream object that
+    ``torch.cuda.current_stream`` makes of it)."""
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
 class _NoGuard:
@@ -231,6 +232,6 @@ def on_device(device: torch.device):
     common case: entering torch.cuda.device costs several microseconds per kernel launch, which
     is most of a decode-sized layer's host time)."""
     index = device.index
-    if index is None or index == torch.cuda.current_device():
+    if index is None or index == torch._C._cuda_getDevice():
         return _NO_GUARD
     return torch.cuda.device(device)

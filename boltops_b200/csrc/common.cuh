@@ -100,6 +100,13 @@ __device__ __forceinline__ int8_t f32_to_i8(float v) {
 int quant_rows(const void* x, int x_dtype, int64_t rows, int cols, int group, int q_dtype, int power2,
                void* q, float* scales, int64_t scales_ld, const int32_t* rows_dev, cudaStream_t st);
 
+// bolt_quant_scatter_rows; without pad_scales the padding positions' scales of the token-order form
+// are left as they are.
+int quant_scatter_rows(const void* x, int x_dtype, int64_t num_tokens, int cols, int group, int q_dtype,
+                       int power2, const int32_t* route_pos, int slots, const int32_t* sorted_ids,
+                       const int32_t* num_valid_ids, int capacity, void* dst, float* dst_scale,
+                       int64_t dst_scale_ld, int codes_in_token_order, int pad_scales, cudaStream_t st);
+
 // 16-byte vector of N elements of T.
 template <typename T, int N>
 struct alignas(sizeof(T) * N) Vec {

@@ -1664,12 +1664,11 @@ extern "C" int bolt_grouped_gemm(const bolt_gemm_args* a, void* stream) {
                                                             : CU_TENSOR_MAP_DATA_TYPE_UINT8;
   const cuuint32_t bk = is16 ? 64 : 128;
   CUtensorMap ma, mb;
-  {
-    // (with a gathered row operand this map is not used by the kernel)
+  memset(&ma, 0, sizeof(ma));
+  if (!gather && !stream_weights) {   // (else the kernel does not use this map)
     // (rows past the end of a dense operand read as zeros)
-    cuuint64_t dims[2] = {(cuuint64_t)a->k, (cuuint64_t)(gather ? a->a_rows : rows)};
-    cuuint64_t strides[1] = {gather && a->a_row_bytes > 0 ? (cuuint64_t)a->a_row_bytes
-                                                          : (cuuint64_t)a->k * elem};
+    cuuint64_t dims[2] = {(cuuint64_t)a->k, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)a->k * elem};
     cuuint32_t box[2] = {bk, (cuuint32_t)kBM};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = encode(&ma, dt, 2, const_cast<void*>(a->a), dims, strides, box, estr,

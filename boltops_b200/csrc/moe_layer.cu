@@ -176,9 +176,9 @@ extern "C" int bolt_moe_layer(const bolt_layer_args* a, void* stream) {
   void* a1 = ws + p.off_a1;
   float* a1_scale = p.quant ? f32(p.off_a1_scale) : nullptr;
   if (p.block) {
-    rc = bolt_quant_scatter_rows(a->hidden_states, a->x_dtype, a->num_tokens, a->hidden, 128,
-                                 q_dtype, 0, route_pos, a->topk, sorted_ids, num_valid, p.cap, a1,
-                                 a1_scale, p.cap, p.gather ? 1 : 0, stream);
+    rc = quant_scatter_rows(a->hidden_states, a->x_dtype, a->num_tokens, a->hidden, 128, q_dtype, 0,
+                            route_pos, a->topk, sorted_ids, num_valid, p.cap, a1, a1_scale, p.cap,
+                            p.gather ? 1 : 0, 0, static_cast<cudaStream_t>(stream));
   } else if (p.quant) {
     rc = bolt_quant_rows(a->hidden_states, a->x_dtype, a->num_tokens, a->hidden, a->hidden,
                          q_dtype, 0, ws + p.off_xq, f32(p.off_xq_scale), 0, stream);

@@ -406,7 +406,7 @@ __device__ __forceinline__ void zero_pad_rows(const int32_t* __restrict__ sorted
                                               int64_t num_tokens, int valid, int row_vecs,
                                               int groups, QTy* __restrict__ dst,
                                               float* __restrict__ dst_scale, int64_t dst_scale_ld,
-                                              int pad_warp, int pad_warps) {
+                                              int pad_warp, int pad_warps, bool token_order) {
   using VOut = Vec<QTy, VEC>;
   const int lane = threadIdx.x & 31;
   VOut zero;
@@ -419,8 +419,10 @@ __device__ __forceinline__ void zero_pad_rows(const int32_t* __restrict__ sorted
     while (mask) {
       const int r = row0 + __ffs(mask) - 1;
       mask &= mask - 1;
-      VOut* d = reinterpret_cast<VOut*>(dst) + (int64_t)r * row_vecs;
-      for (int i = lane; i < row_vecs; i += 32) d[i] = zero;
+      if (!token_order) {   // (else the codes live in token order)
+        VOut* d = reinterpret_cast<VOut*>(dst) + (int64_t)r * row_vecs;
+        for (int i = lane; i < row_vecs; i += 32) d[i] = zero;
+      }
       for (int g = lane; g < groups; g += 32) dst_scale[(int64_t)g * dst_scale_ld + r] = 0.f;
     }
   }
@@ -433,12 +435,12 @@ __device__ __forceinline__ void zero_pad_rows(const int32_t* __restrict__ sorted
 // activations never exist in token order; a token without any such row is not read.  The tail of
 // the kernel zero-fills the rows below num_valid that hold no token (tile padding).
 // token_order: the codes go to token order (the GEMM gathers its rows itself and reads zeros for
-// padding positions) and only the scales to the sorted positions.  What a padding row is scaled by is
-// then nobody's business -- every result of the GEMM depends on its own row alone, and padding rows
-// are not stored -- so it is left unwritten: at three rows per expert those words were 40 times the
-// used ones, one 32-byte sector each.  Measured, DeepSeek-V3 (56 groups, 256 experts), 96 tokens 28.9 ->
-// 3.5 us, one token 10.4 -> 2.9 us; sorted order with 7/8 of the experts elsewhere, 16384 tokens,
-// 127 -> 116 us.
+// padding positions) and only the scales to the sorted positions; padding rows get zero scales only
+// where the caller asks for them.  A layer does not: each result of a GEMM depends on its own row
+// alone and padding rows are not stored, while at three rows per expert there are 40 such words for
+// every used one, a 32-byte sector each.  Measured, DeepSeek-V3 (56 groups, 256 experts), 96 tokens
+// 28.9 -> 3.5 us, one token 10.4 -> 2.9 us; sorted order with 7/8 of the experts elsewhere, 16384
+// tokens, 127 -> 116 us.
 template <typename TIn, int QT, bool POW2, int W>
 __global__ void __launch_bounds__(256) k_quant_scatter(
     const TIn* __restrict__ x, int64_t num_tokens, int cols, int tpg,
@@ -510,7 +512,7 @@ __global__ void __launch_bounds__(256) k_quant_scatter(
   zero_pad_rows<typename QTraits<QT>::type, EPT>(
       sorted_ids, num_tokens, min(*num_valid, capacity), row_units, row_units / tpg, dst,
       dst_scale, dst_scale_ld, (int)(blockIdx.x - quant_blocks) * 8 + (threadIdx.x >> 5),
-      pad_blocks * 8);
+      pad_blocks * 8, token_order != 0);
 }
 
 // Same for groups that span up to 8 x 32 vectors (per-token quantisation of mid-sized rows): one
@@ -583,17 +585,19 @@ __global__ void __launch_bounds__(256) k_quant_scatter_warp(
   const int pad_blocks = gridDim.x - quant_blocks;
   zero_pad_rows<typename QTraits<QT>::type, VEC>(
       sorted_ids, num_tokens, min(*num_valid, capacity), row_vecs, groups, dst, dst_scale,
-      dst_scale_ld, ((int)blockIdx.x - quant_blocks) * 8 + (threadIdx.x >> 5), pad_blocks * 8);
+      dst_scale_ld, ((int)blockIdx.x - quant_blocks) * 8 + (threadIdx.x >> 5), pad_blocks * 8,
+      token_order != 0);
 }
 
 template <typename TIn, int QT, bool POW2>
 int launch_quant_scatter(const void* x, int64_t num_tokens, int cols, int group,
                          const int32_t* route_pos, int slots, const int32_t* sorted_ids,
                          const int32_t* num_valid, int capacity, void* dst, float* dst_scale,
-                         int64_t dst_scale_ld, int token_order, cudaStream_t st) {
+                         int64_t dst_scale_ld, int token_order, int pad_scales, cudaStream_t st) {
   constexpr int VEC = 16 / sizeof(TIn);
   const int tpg = group / VEC;
-  const int pad_blocks = token_order ? 0 : sm_count_of_current_device() * 4;
+  const int pad_blocks = token_order ? (pad_scales ? sm_count_of_current_device() / 2 : 0)
+                                     : sm_count_of_current_device() * 4;
   if (tpg > 32 || (tpg & (tpg - 1)) != 0) {
     // a warp per group, groups strided over a capped grid
     const int64_t num_groups = num_tokens * (cols / group);
@@ -635,7 +639,7 @@ int dispatch_quant_scatter(const void* x, int64_t num_tokens, int cols, int grou
                            int power2, const int32_t* route_pos, int slots,
                            const int32_t* sorted_ids, const int32_t* num_valid, int capacity,
                            void* dst, float* dst_scale, int64_t dst_scale_ld, int token_order,
-                           cudaStream_t st) {
+                           int pad_scales, cudaStream_t st) {
   constexpr int VEC = 16 / sizeof(TIn);
   const int tpg = group / VEC;
   BOLT_REQUIRE(group % VEC == 0 && tpg >= 1 && tpg <= 8 * 32,
@@ -644,7 +648,7 @@ int dispatch_quant_scatter(const void* x, int64_t num_tokens, int cols, int grou
 #define BOLT_QS(QT, P2)                                                                         \
   return launch_quant_scatter<TIn, QT, P2>(x, num_tokens, cols, group, route_pos, slots,        \
                                            sorted_ids, num_valid, capacity, dst, dst_scale,     \
-                                           dst_scale_ld, token_order, st)
+                                           dst_scale_ld, token_order, pad_scales, st)
   if (q_dtype == BOLT_FP8_E4M3) {
     if (power2) BOLT_QS(BOLT_FP8_E4M3, true);
     BOLT_QS(BOLT_FP8_E4M3, false);
@@ -851,15 +855,12 @@ extern "C" int bolt_gather_rows(const void* src, int num_tokens, int row_bytes,
   return BOLT_OK;
 }
 
-extern "C" int bolt_quant_scatter_rows(const void* x, int x_dtype, int64_t num_tokens, int cols,
-                                       int group, int q_dtype, int power2,
-                                       const int32_t* route_pos, int slots,
-                                       const int32_t* sorted_ids, const int32_t* num_valid_ids,
-                                       int capacity, void* dst, float* dst_scale,
-                                       int64_t dst_scale_ld, int codes_in_token_order,
-                                       void* stream) {
+int bolt::quant_scatter_rows(const void* x, int x_dtype, int64_t num_tokens, int cols, int group,
+                             int q_dtype, int power2, const int32_t* route_pos, int slots,
+                             const int32_t* sorted_ids, const int32_t* num_valid_ids, int capacity,
+                             void* dst, float* dst_scale, int64_t dst_scale_ld,
+                             int codes_in_token_order, int pad_scales, cudaStream_t st) {
   using namespace bolt;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   BOLT_REQUIRE(num_tokens >= 0 && cols > 0 && capacity >= 0 && slots > 0,
                "quant_scatter: bad shape");
   BOLT_REQUIRE(group > 0 && cols % group == 0, "quant_scatter: group %d does not divide cols %d",
@@ -880,19 +881,31 @@ extern "C" int bolt_quant_scatter_rows(const void* x, int x_dtype, int64_t num_t
       return dispatch_quant_scatter<__nv_bfloat16>(x, num_tokens, cols, group, q_dtype, power2,
                                                    route_pos, slots, sorted_ids, num_valid_ids,
                                                    capacity, dst, dst_scale, dst_scale_ld,
-                                                   codes_in_token_order, st);
+                                                   codes_in_token_order, pad_scales, st);
     case BOLT_F16:
       return dispatch_quant_scatter<__half>(x, num_tokens, cols, group, q_dtype, power2,
                                             route_pos, slots, sorted_ids, num_valid_ids, capacity,
-                                            dst, dst_scale, dst_scale_ld, codes_in_token_order, st);
+                                            dst, dst_scale, dst_scale_ld, codes_in_token_order, pad_scales, st);
     case BOLT_F32:
       return dispatch_quant_scatter<float>(x, num_tokens, cols, group, q_dtype, power2, route_pos,
                                            slots, sorted_ids, num_valid_ids, capacity, dst,
-                                           dst_scale, dst_scale_ld, codes_in_token_order, st);
+                                           dst_scale, dst_scale_ld, codes_in_token_order, pad_scales, st);
     default:
       set_error("quant_scatter: unsupported input dtype %d", x_dtype);
       return BOLT_ERR_INVALID;
   }
+}
+
+extern "C" int bolt_quant_scatter_rows(const void* x, int x_dtype, int64_t num_tokens, int cols,
+                                       int group, int q_dtype, int power2,
+                                       const int32_t* route_pos, int slots,
+                                       const int32_t* sorted_ids, const int32_t* num_valid_ids,
+                                       int capacity, void* dst, float* dst_scale,
+                                       int64_t dst_scale_ld, int codes_in_token_order,
+                                       void* stream) {
+  return bolt::quant_scatter_rows(x, x_dtype, num_tokens, cols, group, q_dtype, power2, route_pos, slots,
+                                  sorted_ids, num_valid_ids, capacity, dst, dst_scale, dst_scale_ld,
+                                  codes_in_token_order, 1, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int bolt_mx_quant_rows(const void* x, int x_dtype, int64_t rows, int cols, int gated,

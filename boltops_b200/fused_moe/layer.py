@@ -287,7 +287,7 @@ def fused_experts_impl(
     for what, cols, esz in (("hidden size", w1.shape[2], w1.element_size()),
                             ("intermediate size", w2.shape[2], w2.element_size()),
                             ("hidden size", w1.shape[2], hidden_states.element_size()),
-                            ("output size", w2.shape[1], torch.empty((), dtype=output_dtype).element_size())):
+                            ("output size", w2.shape[1], output_dtype.itemsize)):
         if (cols * esz) % 16:
             raise NotImplementedError(
                 f"{what} {cols} x {esz} B is not a multiple of 16 bytes: not built in boltops_b200")

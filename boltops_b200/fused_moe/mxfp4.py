@@ -213,6 +213,7 @@ def fused_experts_mxfp4(hidden_states, w1, w2, topk_weights, topk_ids, *, w1_sca
     native = (_NATIVE and not static and hidden_states.dtype != torch.float8_e4m3fn
               and w1.is_contiguous() and w2.is_contiguous()
               and w1.data_ptr() % 32 == 0 and w2.data_ptr() % 32 == 0)
+    from .layer import _use_gather
     if native:
         from .mxfp8 import _tile_weight_scales
         fuse_act = _FUSED and activation == "silu" and inter % 128 == 0
@@ -262,19 +263,21 @@ def fused_experts_mxfp4(hidden_states, w1, w2, topk_weights, topk_ids, *, w1_sca
         if expert_map is not None:
             expert_ids = ops.relabel_tiles(expert_ids, expert_map)
         cap = sorted_ids.shape[0]
-        a_sorted, _ = ops.gather_rows(a_tok, sorted_ids, num_valid, cap)
+        # (the native GEMM1 gathers the codes itself while sorted rows would be mostly padding)
+        in_gemm = native and _use_gather(m * topk, global_num_experts)
+        a1 = a_tok if in_gemm else ops.gather_rows(a_tok, sorted_ids, num_valid, cap)[0]
         common = dict(kind=_cabi.GEMM_MXFP4 if native else _cabi.GEMM_BF16,
                       sorted_expert_ids=expert_ids, num_valid=num_valid,
                       sorted_ids=sorted_ids, sorted_weights=sorted_w, num_tokens=m, topk=topk)
         if native:
-            gemm1 = dict(b=w1, a_scale=ops.mx_sf_layout(a_sf, cap, sorted_ids, num_valid),
+            gemm1 = dict(a=a1, a_gather=in_gemm, b=w1, a_scale=ops.mx_sf_layout(a_sf, cap, sorted_ids, num_valid),
                          b_scale=sfb1)
         else:
-            gemm1 = dict(b=w1_d)
+            gemm1 = dict(a=a1, b=w1_d)
         # ---- GEMM1, activation, second quantisation ------------------------------------------
         if static:
             g1 = torch.empty((cap, n1), device=dev, dtype=torch.float32)
-            ops.grouped_gemm(epilogue=_cabi.EPI_STORE, a=a_sorted, b=w1_d, c=g1, **common)
+            ops.grouped_gemm(epilogue=_cabi.EPI_STORE, a=a1, b=w1_d, c=g1, **common)
             act = torch.empty((cap, inter), device=dev, dtype=torch.bfloat16)
             with _cabi.on_device(dev):
                 check(lib.bolt_mx4_swiglu_static(
@@ -288,13 +291,13 @@ def fused_experts_mxfp4(hidden_states, w1, w2, topk_weights, topk_ids, *, w1_sca
             # 1 x 128 power-of-two quantiser; codes and exponent bytes go straight to GEMM2
             act = torch.empty((cap, inter), device=dev, dtype=torch.float8_e4m3fn)
             act_s = torch.empty((cap, inter // 32), device=dev, dtype=torch.uint8)
-            ops.grouped_gemm(epilogue=_cabi.EPI_SILU_MUL_QUANT, a=a_sorted, c=act, c_scale=act_s,
+            ops.grouped_gemm(epilogue=_cabi.EPI_SILU_MUL_QUANT, c=act, c_scale=act_s,
                              c_scale_ld=inter // 32, mid_dtype=out_dtype, act_limit=limit,
                              **gemm1, **common)
             gemm2 = dict(a=act, b=w2, a_scale=ops.mx_sf_layout(act_s, cap), b_scale=sfb2)
         else:
             g1 = torch.empty((cap, n1), device=dev, dtype=out_dtype)
-            ops.grouped_gemm(epilogue=_cabi.EPI_STORE, a=a_sorted, c=g1, **gemm1, **common)
+            ops.grouped_gemm(epilogue=_cabi.EPI_STORE, c=g1, **gemm1, **common)
             want = dict(want_codes=True, want_deq=False, want_sf=True) if native else {}
             if activation == "silu":
                 q2 = act_quant(g1, gated=True, limit=limit, **want)

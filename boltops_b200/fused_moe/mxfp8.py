@@ -154,6 +154,7 @@ def fused_experts_mxfp8(hidden_states, w1, w2, topk_weights, topk_ids, *, w1_sca
     # itself (BOLT_GEMM_MXFP8) and the weights stay in 8 bits.  Otherwise the operands are
     # dequantised (exactly) and the 16-bit kind computes the same contraction.
     native = hidden % 128 == 0 and inter % 128 == 0
+    from .layer import _use_gather
     if native:
         kind = _cabi.GEMM_MXFP8
         w1 = w1 if w1.is_contiguous() else w1.contiguous()
@@ -191,19 +192,21 @@ def fused_experts_mxfp8(hidden_states, w1, w2, topk_weights, topk_ids, *, w1_sca
         common = dict(kind=kind, sorted_expert_ids=expert_ids, num_valid=num_valid,
                       sorted_ids=sorted_ids, sorted_weights=sorted_w, num_tokens=m, topk=topk)
         if native:
-            # A1: codes + exponent bytes once per token; codes gathered into sorted rows, bytes
-            # gathered straight into the tiled layout
+            # A1: codes + exponent bytes once per token; codes gathered into sorted rows, or by GEMM1
+            # itself while those rows would be mostly padding (layer._use_gather); bytes gathered
+            # straight into the tiled layout
+            in_gemm = _use_gather(m * topk, global_num_experts)
             with _Stage("quant_a1"):
                 x_q, x_s, _ = ops.mx_quant_rows(hidden_states[begin:end])
             with _Stage("gather"):
-                a_sorted, _ = ops.gather_rows(x_q, sorted_ids, num_valid, cap)
+                a1 = x_q if in_gemm else ops.gather_rows(x_q, sorted_ids, num_valid, cap)[0]
                 sfa = ops.mx_sf_layout(x_s, cap, sorted_ids, num_valid)
             # GEMM1 with the rounding to the input dtype, the split gated activation (fp32) and
             # the second quantisation in its epilogue: 32 outputs of a thread are one MX group
             act = torch.empty((cap, inter), device=dev, dtype=torch.float8_e4m3fn)
             act_s = torch.empty((cap, inter // 32), device=dev, dtype=torch.uint8)
             with _Stage("gemm1"):
-                ops.grouped_gemm(epilogue=_cabi.EPI_SILU_MUL_QUANT, a=a_sorted, b=w1, c=act,
+                ops.grouped_gemm(epilogue=_cabi.EPI_SILU_MUL_QUANT, a=a1, a_gather=in_gemm, b=w1, c=act,
                                  a_scale=sfa, b_scale=sfb1, c_scale=act_s,
                                  c_scale_ld=inter // 32, mid_dtype=dtype, act_alpha=alpha,
                                  act_beta=beta, act_limit=gemm1_limit, **common)

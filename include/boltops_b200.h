@@ -504,7 +504,7 @@ typedef struct bolt_gemm_args {
   int max_segments;
   const int32_t* segments;
   const int32_t* num_segments;
-  /* Gathered row operand (plain kinds, single-tile schedule).  With a_gather != 0, `a` is NOT in
+  /* Gathered row operand (single-tile schedule).  With a_gather != 0, `a` is NOT in
      sorted order: it is the token-order matrix [a_rows >= num_tokens, k] (a_row_bytes between
      rows, a multiple of 16; 0 = dense), and sorted position p reads row sorted_ids[p] & 0xFFFFFF,
      or zeros where that id is not a token (id >= num_tokens: tile padding).  a_scale stays in

@@ -38,16 +38,22 @@ def gemm_a8w8_blockscale(x: torch.Tensor, w: torch.Tensor, x_scale: torch.Tensor
         raise ValueError("scale shapes do not match the 1x128 / 128x128 recipe")
     kind = _cabi.GEMM_FP8_BLOCK if x.dtype == torch.float8_e4m3fn else _cabi.GEMM_INT8_BLOCK
     dev = x.device
+    # the kernels take addresses: none of another device may reach them
+    for name, t in (("w", w), ("w_scale", w_scale)):
+        if t.device != dev:
+            raise ValueError(f"{name} is on {t.device}, x on {dev}")
     if out is not None:
         assert out.shape == (m, n) and out.dtype == dtype and out.is_contiguous()
-    c = out if out is not None else torch.empty((m, n), dtype=dtype, device=dev)
+    elsewhere = out is not None and out.device != dev     # the result is copied there
+    c = out if out is not None and not elsewhere else torch.empty((m, n), dtype=dtype, device=dev)
     if m == 0:
-        return c
+        return out if elsewhere else c
     # Two launches: the scales to group-major order (with the one "expert"'s tile labels), the GEMM.
     # Rows that only pad the last row tile exist nowhere: the tensor map reads them as zeros and
     # nothing is stored for them.
     x, w = x.contiguous(), w.contiguous()
-    x_scale, w_scale = x_scale.float().contiguous(), w_scale.float().contiguous()
+    x_scale = x_scale.to(device=dev, dtype=torch.float32).contiguous()
+    w_scale = w_scale.float().contiguous()
     cap = ops.ceil_to(m, 128)
     groups, tiles = k // 128, cap // 128
     ws = torch.empty(groups * cap + tiles + 1, dtype=torch.float32, device=dev)
@@ -72,6 +78,8 @@ def gemm_a8w8_blockscale(x: torch.Tensor, w: torch.Tensor, x_scale: torch.Tensor
                                         num_rows, stream))
         _cabi.check(lib.bolt_grouped_gemm(args, stream))
     ops._count(2)
+    if elsewhere:
+        return out.copy_(c)
     return c
 
 

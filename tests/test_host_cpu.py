@@ -235,3 +235,46 @@ def test_gathered_row_operand_rule_and_layer_kernel_count(monkeypatch):
     assert fp8 >= 5 and count(_cabi.GEMM_INT8_CHANNEL, 16) == fp8 + 2
     bad = _cabi.LayerArgs()
     assert lib.bolt_moe_layer_kernel_count(bad) == -1
+
+
+class _OnGpu(torch.Tensor):
+    """Passes for a GPU tensor, so that the host side of a call can be followed here."""
+    is_cuda = True
+
+
+def test_dense_gemm_hands_the_kernels_no_address_of_another_device(monkeypatch):
+    """The operands' devices are settled before any launch: weights and their scales elsewhere are
+    refused, scales of the rows are brought along, a result wanted elsewhere is copied there."""
+    from boltops_b200 import _cabi, gemm
+    seen = []
+
+    class Lib:
+        def bolt_dense_prep(self, scale, *rest):
+            seen.append(("scale", scale))
+            return 0
+
+        def bolt_grouped_gemm(self, args, stream):
+            seen.append(("gemm", args.a, args.c))
+            return 0
+
+    monkeypatch.setattr(_cabi, "load", lambda: Lib())
+    monkeypatch.setattr(_cabi, "stream_of", lambda t: 0)
+    monkeypatch.setattr(gemm.ops, "device_status", lambda d: torch.zeros(1, dtype=torch.int32))
+    m, n, k = 3, 128, 256
+    flat = torch.zeros(m * k + 16, dtype=torch.int8)
+    skip = -flat.data_ptr() % 16
+    x = flat[skip:skip + m * k].view(m, k).as_subclass(_OnGpu)
+    w = torch.zeros(n, k, dtype=torch.int8)
+    xs, ws = torch.ones(m, k // 128), torch.ones(n // 128, k // 128)
+
+    for bad in (dict(w=w.to("meta")), dict(w_scale=ws.to("meta"))):
+        with pytest.raises(ValueError, match="x on cpu"):
+            gemm.gemm_a8w8_blockscale(x, bad.get("w", w), xs, bad.get("w_scale", ws))
+    assert not seen
+
+    gemm.gemm_a8w8_blockscale(x, w, xs, ws)
+    assert [s[0] for s in seen] == ["scale", "gemm"] and seen[1][1] == x.data_ptr()
+    seen.clear()
+    out = torch.empty(m, n, dtype=torch.bfloat16, device="meta")
+    assert gemm.gemm_a8w8_blockscale(x, w, xs, ws, out=out) is out
+    assert seen[1][2] not in (0, None)      # a buffer of x's device, not the address of `out`

@@ -52,3 +52,21 @@ def test_dense_rows_end_inside_a_tile(dtype, m, n, k):
     assert (buf[m:] == -7.0).all()
     some = gemm_a8w8_blockscale(x[:m], w, xs[:m].double(), ws, dtype=dtype)   # any floating scale type
     assert torch.equal(some.cpu(), out.cpu())
+
+
+def test_dense_operands_off_the_device():
+    """Row scales and the result may lie in host memory."""
+    from boltops_b200.gemm import gemm_a8w8_blockscale
+    m, n, k = 130, 128, 256
+    g = torch.Generator().manual_seed(2)
+    x = torch.randint(-127, 128, (m, k), generator=g, dtype=torch.int8)
+    w = torch.randint(-127, 128, (n, k), generator=g, dtype=torch.int8).cuda()
+    xs, ws = torch.rand(m, k // 128, generator=g), torch.rand(n // 128, k // 128, generator=g).cuda()
+    want = gemm_a8w8_blockscale(x.cuda(), w, xs.cuda(), ws)
+    assert torch.equal(gemm_a8w8_blockscale(x.cuda(), w, xs, ws), want)
+    host = torch.zeros(m, n, dtype=torch.bfloat16)
+    assert gemm_a8w8_blockscale(x.cuda(), w, xs.cuda(), ws, out=host) is host
+    assert torch.equal(host, want.cpu())
+    for moved in (dict(w=w.cpu()), dict(w_scale=ws.cpu())):
+        with pytest.raises(ValueError, match="x on cuda"):
+            gemm_a8w8_blockscale(x.cuda(), moved.get("w", w), xs.cuda(), moved.get("w_scale", ws))

@@ -52,6 +52,8 @@ def gemm_a8w8_blockscale(x: torch.Tensor, w: torch.Tensor, x_scale: torch.Tensor
     # Rows that only pad the last row tile exist nowhere: the tensor map reads them as zeros and
     # nothing is stored for them.
     x, w = x.contiguous(), w.contiguous()
+    if x.data_ptr() % 16:
+        x = x.clone()       # the tensor map needs a 16-byte aligned base
     x_scale = x_scale.to(device=dev, dtype=torch.float32).contiguous()
     w_scale = w_scale.float().contiguous()
     cap = ops.ceil_to(m, 128)

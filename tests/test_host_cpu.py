@@ -243,8 +243,9 @@ class _OnGpu(torch.Tensor):
 
 
 def test_dense_gemm_hands_the_kernels_no_address_of_another_device(monkeypatch):
-    """The operands' devices are settled before any launch: weights and their scales elsewhere are
-    refused, scales of the rows are brought along, a result wanted elsewhere is copied there."""
+    """The operands' devices and the row operand's alignment are settled before any launch: weights
+    and their scales elsewhere are refused, scales of the rows are brought along, a result wanted
+    elsewhere is copied there, and a row operand off the 16-byte grid is copied once."""
     from boltops_b200 import _cabi, gemm
     seen = []
 
@@ -274,6 +275,10 @@ def test_dense_gemm_hands_the_kernels_no_address_of_another_device(monkeypatch):
 
     gemm.gemm_a8w8_blockscale(x, w, xs, ws)
     assert [s[0] for s in seen] == ["scale", "gemm"] and seen[1][1] == x.data_ptr()
+    seen.clear()
+    odd = flat[skip + 1:skip + 1 + m * k].view(m, k).as_subclass(_OnGpu)
+    gemm.gemm_a8w8_blockscale(odd, w, xs, ws)
+    assert seen[1][1] % 16 == 0 and seen[1][1] != odd.data_ptr()
     seen.clear()
     out = torch.empty(m, n, dtype=torch.bfloat16, device="meta")
     assert gemm.gemm_a8w8_blockscale(x, w, xs, ws, out=out) is out

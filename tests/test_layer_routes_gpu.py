@@ -54,8 +54,8 @@ def test_dense_rows_end_inside_a_tile(dtype, m, n, k):
     assert torch.equal(some.cpu(), out.cpu())
 
 
-def test_dense_operands_off_the_device():
-    """Row scales and the result may lie in host memory."""
+def test_dense_operands_off_the_device_or_the_16_byte_grid():
+    """Row scales and the result may lie in host memory, x and the result at any address."""
     from boltops_b200.gemm import gemm_a8w8_blockscale
     m, n, k = 130, 128, 256
     g = torch.Generator().manual_seed(2)
@@ -67,6 +67,14 @@ def test_dense_operands_off_the_device():
     host = torch.zeros(m, n, dtype=torch.bfloat16)
     assert gemm_a8w8_blockscale(x.cuda(), w, xs.cuda(), ws, out=host) is host
     assert torch.equal(host, want.cpu())
+    odd = torch.zeros(m * k + 1, dtype=torch.int8, device="cuda")[1:].view(m, k)
+    odd.copy_(x)
+    assert torch.equal(gemm_a8w8_blockscale(odd, w, xs.cuda(), ws), want)
+    for dtype in (torch.bfloat16, torch.float32):
+        buf = torch.zeros(m * n + 1, dtype=dtype, device="cuda")
+        out = buf[1:].view(m, n)
+        gemm_a8w8_blockscale(x.cuda(), w, xs.cuda(), ws, dtype=dtype, out=out)
+        assert torch.equal(out, gemm_a8w8_blockscale(x.cuda(), w, xs.cuda(), ws, dtype=dtype))
     for moved in (dict(w=w.cpu()), dict(w_scale=ws.cpu())):
         with pytest.raises(ValueError, match="x on cuda"):
             gemm_a8w8_blockscale(x.cuda(), moved.get("w", w), xs.cuda(), moved.get("w_scale", ws))

@@ -41,12 +41,15 @@ using namespace tc;
 constexpr int kThreads = 384;
 // Shared-memory operand stages against bulk-store slots.  The block-scaled kinds spend ~950 cycles
 // per K block, three stages cover the load latency, and the space goes to the slots.  The other
-// 8-bit kinds stream a K block every ~500 cycles; their down projection runs a short reduction,
-// so that the stores are the longer half of a tile, and takes the same division (Qwen3-30B int8,
-// 16384 tokens, K = 768: 284 us with one slot per warp, 232 us with four).  Their gated GEMM and the
-// 16-bit kinds keep four stages (same layer, K = 2048: 366 us against 381 us with three).
-constexpr bool more_slots(int opk, bool block_scaled, int epi) {
-  return block_scaled || (opk != OP_F16 && epi == BOLT_EPI_STORE);
+// kinds stream a K block every ~500 cycles and want four stages, except where the reduction is so
+// short that the stores are the longer half of a tile: single tiles of the 8-bit kinds with a plain
+// epilogue and at most kShortK columns.  Measured, four stages -> three, in us: 128 experts x 1024
+// rows x 2048, int8, K = 256 190 -> 185, K = 512 229 -> 212, K = 768 263 -> 277, K = 2048 558 -> 592; e4m3
+// 32 x 2048 x 4096, K = 512 302 -> 248, K = 768 253 -> 286; 64 x 96 x 4096, int8, K = 512 56 -> 44.
+// At K = 640 either may win by 5 %.  Gated (Qwen3-30B, K = 2048) 366 -> 381; tile pairs gain nothing.
+constexpr int kShortK = 512;
+constexpr bool short_k_form(int opk, bool block_scaled, int epi, bool pair) {
+  return !block_scaled && opk != OP_F16 && epi == BOLT_EPI_STORE && !pair;
 }
 constexpr int stages_of(bool slots) { return slots ? 3 : 4; }
 constexpr int kBM = 128;
@@ -465,12 +468,11 @@ __device__ __forceinline__ void gather_row_tiles(const GemmParams& p, uint32_t s
 // "full" barrier; MMA completion is committed to both CTAs' "empty" / "tfull" barriers; the odd
 // CTA's epilogue warps release TMEM stages on the even CTA's "tempty" barrier.  No load is
 // multicast.
-template <int OPK, bool BS, int EPI, bool PAIR>
+template <int OPK, bool BS, int EPI, bool PAIR, bool MORE_SLOTS>
 __global__ void __launch_bounds__(kThreads, 1)
 k_grouped_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                const __grid_constant__ CUtensorMap tma_c, const GemmParams p) {
   constexpr bool GATED = EPI != BOLT_EPI_STORE;
-  constexpr bool MORE_SLOTS = more_slots(OPK, BS, EPI);
   constexpr int kBKElems = OPK == OP_F16 ? 64 : 128;
   constexpr bool CHANNEL = (OPK != OP_F16) && !BS;
   constexpr int kStages = PAIR ? pair_stages_of(MORE_SLOTS) : stages_of(MORE_SLOTS);
@@ -1511,11 +1513,10 @@ EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-template <int OPK, bool BS, int EPI, bool PAIR>
-int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc,
-           const GemmParams& p, int grid, cudaStream_t st) {
-  auto kfn = k_grouped_gemm<OPK, BS, EPI, PAIR>;
-  constexpr bool slots = more_slots(OPK, BS, EPI);
+template <int OPK, bool BS, int EPI, bool PAIR, bool slots>
+int launch_form(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc,
+                const GemmParams& p, int grid, cudaStream_t st) {
+  auto kfn = k_grouped_gemm<OPK, BS, EPI, PAIR, slots>;
   constexpr int smem = PAIR ? pair_smem_bytes_of(slots) : smem_bytes_of(slots);
   static std::atomic<bool> configured[kMaxDevices];
   // warps 0-3 drop to 56 registers, the eight epilogue warps rise to 224
@@ -1540,6 +1541,15 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc,
   }
   BOLT_LAUNCH_CHECK();
   return BOLT_OK;
+}
+
+template <int OPK, bool BS, int EPI, bool PAIR>
+int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc,
+           const GemmParams& p, int grid, cudaStream_t st) {
+  if constexpr (short_k_form(OPK, BS, EPI, PAIR)) {
+    if (p.k <= kShortK) return launch_form<OPK, BS, EPI, PAIR, true>(ma, mb, mc, p, grid, st);
+  }
+  return launch_form<OPK, BS, EPI, PAIR, BS>(ma, mb, mc, p, grid, st);
 }
 
 template <int OPK, bool BS, bool PAIR>

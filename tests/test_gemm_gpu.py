@@ -417,3 +417,44 @@ def test_gemm_gathered_rows_with_reduction_and_column_tails():
         ops.check_device_status(c.device)
         outs.append(c)
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("k", [128, 384, 512])     # up to 512: three operand stages, four store slots
+@pytest.mark.parametrize("n", [256, 296])          # 296: a last column tile that is part empty
+@pytest.mark.parametrize("c_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("scatter", [False, True])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_per_channel_short_reduction(fp8, scatter, c_dtype, n, k):
+    """Columns of zeros that carry the reduction past 512 change the division of shared memory and
+    nothing else: equal bit for bit.  Three CTAs, so that each takes several tiles in a row."""
+    from boltops_b200 import _cabi
+    from boltops_b200.fused_moe import ops
+    e, m, topk = 4, 300, 2
+    dt = torch.float8_e4m3fn if fp8 else torch.int8
+    g = torch.Generator().manual_seed(k + n)
+    ids = torch.stack([torch.randperm(e, generator=g)[:topk] for _ in range(m)]).to(torch.int32)
+    wts = torch.rand(m, topk, generator=g).cuda()
+    sorted_ids, sorted_w, expert_ids, num_valid = ops.moe_sorting_ck(
+        ids.cuda(), wts, e, None, None, 128, None, alloc_moe_buf=False)[:4]
+    cap = sorted_ids.shape[0]
+    a = torch.randint(-127, 128, (cap, k), generator=g).float().to(dt).cuda()
+    b = torch.randint(-127, 128, (e, n, k), generator=g).float().to(dt).cuda()
+    a_s, b_s = torch.rand(cap, generator=g).cuda(), torch.rand(e, n, generator=g).cuda()
+    bias = torch.randn(e, n, generator=g).cuda()
+    outs = []
+    for width in (k, 640):
+        rows, cols = torch.zeros(cap, width, dtype=dt), torch.zeros(e, n, width, dtype=dt)
+        rows[:, :k], cols[:, :, :k] = a.cpu(), b.cpu()
+        c = torch.zeros(m * topk if scatter else cap, n, dtype=c_dtype, device="cuda")
+        ops.grouped_gemm(kind=_cabi.GEMM_FP8_CHANNEL if fp8 else _cabi.GEMM_INT8_CHANNEL,
+                         epilogue=_cabi.EPI_STORE, a=rows.cuda(), b=cols.cuda(), c=c,
+                         sorted_expert_ids=expert_ids, num_valid=num_valid, a_scale=a_s,
+                         a_scale_ld=cap, b_scale=b_s, bias=bias, scatter=scatter, num_tokens=m,
+                         topk=topk, mul_routed_weight=True, sorted_ids=sorted_ids,
+                         sorted_weights=sorted_w, sm_count=3)
+        live = (sorted_ids & 0xFFFFFF) < m
+        live[int(num_valid):] = False
+        outs.append((c if scatter else c[live]).cpu())
+    ops.check_device_status(torch.device("cuda", 0))
+    assert torch.isfinite(outs[0]).all() and outs[0].abs().max() > 0
+    assert torch.equal(outs[0], outs[1])

@@ -25,6 +25,8 @@ GEMM_BF16, GEMM_F16, GEMM_FP8_BLOCK, GEMM_INT8_CHANNEL, GEMM_FP8_CHANNEL, GEMM_I
     GEMM_MXFP8, GEMM_MXFP4 = range(8)
 # enum bolt_gemm_epilogue
 EPI_STORE, EPI_SILU_MUL, EPI_SILU_MUL_QUANT = range(3)
+# BOLT_ABI_VERSION of the header these structures were written against
+ABI_VERSION = 4
 # enum bolt_gemm_schedule, BOLT_PAIR_SEGMENT_ROWS
 SCHEDULE_ROW_TILES, SCHEDULE_TILE_PAIRS, SCHEDULE_STREAM = range(3)
 PAIR_SEGMENT_ROWS = 256
@@ -189,7 +191,7 @@ def load() -> C.CDLL:
         fn = getattr(lib, name)
         fn.restype = res
         fn.argtypes = args
-    if lib.bolt_abi_version() != 3:
+    if lib.bolt_abi_version() != ABI_VERSION:
         raise RuntimeError("libboltops_b200.so ABI version mismatch")
     _lib = lib
     return lib

@@ -23,7 +23,7 @@
 extern "C" {
 #endif
 
-#define BOLT_ABI_VERSION 3
+#define BOLT_ABI_VERSION 4
 
 enum bolt_status {
   BOLT_OK = 0,

@@ -30,7 +30,7 @@ def test_library_exports_every_declared_symbol(lib):
     for name in declared:
         assert hasattr(lib, name), f"{name} declared in the header but not exported"
     assert declared == set(_cabi.EXPORTS)
-    assert lib.bolt_abi_version() == 3
+    assert lib.bolt_abi_version() == _cabi.ABI_VERSION == 4
 
 
 def test_gemm_args_struct_matches_header(tmp_path):
@@ -50,6 +50,14 @@ def test_gemm_args_struct_matches_header(tmp_path):
     assert nums[0] == ctypes.sizeof(_cabi.GemmArgs)
     for f, off in zip(fields, nums[1:]):
         assert getattr(_cabi.GemmArgs, f).offset == off, f
+
+
+def test_abi_version_goes_with_the_structures():
+    """Bindings compare the version and then hand over structures of their own: whoever changes a
+    structure's size has to raise the version (and extend this table)."""
+    from boltops_b200 import _cabi
+    sizes = {3: (264, 168), 4: (272, 176)}     # 4: three more fields
+    assert sizes[_cabi.ABI_VERSION] == (ctypes.sizeof(_cabi.GemmArgs), ctypes.sizeof(_cabi.LayerArgs))
 
 
 def test_layer_args_struct_matches_header(tmp_path):

@@ -27,12 +27,19 @@ constexpr int kUnit = 128;
 // sorted layout is mostly tile padding (measured on the DeepSeek-V3 fp8 layer: 0.120 vs 0.152 ms
 // at 8 routes, 0.49 vs 0.52 ms at 16 routes per expert, even at 128, 4.56 vs 4.51 ms at 256
 // routes per expert, where the extra copy instructions slow the accumulator promotion down), so
-// it is used up to kGatherMaxAvgRows routes per expert.  The per-channel kinds have no promotion to
-// slow down, and their rows in token order stay in L2 where the sorted copy does not: there it is
-// used from that size on (Qwen3-30B int8: 16384 tokens, sorted copy + GEMM 1 93 + 363 us, gathered
-// 400 us; 1200 tokens 10 + 87 against 82 us).  BOLTOPS_B200_GATHER=0 / 1 forces it off
-// / on.
+// it is used up to kGatherMaxAvgRows routes per expert.
+// The per-channel kinds have no promotion to slow down, and there the gather spares a pass over
+// codes that the quantiser has just written; it is used above that size, for intermediate sizes up
+// to kGatherMaxInter.  What it costs grows with GEMM 1 (every column tile gathers its rows again),
+// what it spares does not.  Measured on int8 layers, sorted copy / gather in us: hidden x intermediate
+// 2048 x 768, 128 experts, 1040 tokens 170 / 155, 16384 tokens 923 / 871; 7168 x 2048, 64 experts, 1024
+// tokens 668 / 622, 8192 tokens 3147 / 3098; 4096 x 4096, 32 experts, 2048 tokens 558 / 569, 16384
+// tokens 3358 / 3464; 2048 x 8192, 16 experts, 16384 tokens 1647 / 1783; 4096 x 14336, 8 experts, 1024
+// tokens 502 / 518, 4096 tokens 1384 / 1550.  At 64 routes per expert and fewer, where the streaming
+// schedule runs up to 32, the gather would win as well (16 to 64 routes: 1 to 12 %) and is not used yet.
+// BOLTOPS_B200_GATHER=0 / 1 forces it off / on.
 constexpr int kGatherMaxAvgRows = 64;
+constexpr int kGatherMaxInter = 2048;
 bool gather_rows_in_gemm(const bolt_layer_args* a) {
   static const int forced = [] {
     const char* v = std::getenv("BOLTOPS_B200_GATHER");
@@ -41,7 +48,9 @@ bool gather_rows_in_gemm(const bolt_layer_args* a) {
   }();
   if (forced >= 0) return forced == 1;
   const bool few = (int64_t)a->num_tokens * a->topk <= (int64_t)kGatherMaxAvgRows * a->global_num_experts;
-  return a->kind == BOLT_GEMM_INT8_CHANNEL || a->kind == BOLT_GEMM_FP8_CHANNEL ? !few : few;
+  if (a->kind == BOLT_GEMM_INT8_CHANNEL || a->kind == BOLT_GEMM_FP8_CHANNEL)
+    return !few && a->inter <= kGatherMaxInter;
+  return few;
 }
 
 inline size_t a256(size_t n) { return (n + 255) & ~size_t(255); }

@@ -62,7 +62,9 @@ _ONE_CALL = os.environ.get("BOLTOPS_B200_ONE_CALL", "1") != "0"
 # reading a copy in sorted order; same results.  It wins while the sorted layout is mostly tile
 # padding and loses once experts have more than a tile of rows (the extra copy instructions slow
 # the accumulator promotion down), so it is used up to _GATHER_MAX_AVG_ROWS routes per expert --
-# the rule of bolt_moe_layer.  BOLTOPS_B200_GATHER=0 / 1 forces it off / on.
+# the rule of bolt_moe_layer for these kinds.  Per-channel experts gather in bolt_moe_layer alone (by
+# a rule of its own); driven kernel by kernel they read sorted rows.
+# BOLTOPS_B200_GATHER=0 / 1 forces it off / on.
 _GATHER = {"0": False, "1": True}.get(os.environ.get("BOLTOPS_B200_GATHER", ""), None)
 _GATHER_MAX_AVG_ROWS = 64
 

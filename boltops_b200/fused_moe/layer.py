@@ -121,14 +121,29 @@ def _use_tile_pairs(kind: int, routes: int, experts: int) -> bool:
 _PAIR_MIN_AVG_ROWS = 384
 
 
-def _use_stream(kind: int, routes: int, experts: int, hidden: int, inter: int) -> bool:
+def _use_stream(kind: int, routes: int, experts: int, hidden: int, inter: int,
+                local_experts: Optional[int] = None) -> bool:
     """Whether the two GEMMs run in the weight-streaming form (``csrc/stream_gemm.cuh``), which
     computes only live rows and is bound by HBM up to about 32 of them per expert.  Equal results, so
-    the line is one of speed alone, both sides measured in us per layer (row tiles / streaming).
-    Block-scaled kinds, whose promotion needs a scale per row there: DeepSeek-V3 fp8, 3 routes per
-    expert 1934 / 1877, 8: 2011 / 1985, 16: 2134 / 2121, 50: 308 / 337 (32 experts); Zipf-distributed
-    routing at 16 routes per expert (hot experts of 200) 482 / 472.  The others: Mixtral bf16, 16
-    routes per expert 482 / 461, Qwen3-30B int8, 32: 202 / 191, Mixtral 100: 475 / 621.
+    the line is one of speed alone.  Both sides measured in us per layer, row tiles / streaming,
+    routes per expert in brackets:
+
+    Block-scaled kinds, whose promotion needs a scale per row there, up to 16: DeepSeek-V3 fp8 with
+    32 experts [8] 299 / 253, [16] 308 / 266, [32] 310 / 296; with 256 [16] 2138 / 2082, [24] 2161 /
+    2115; Qwen3-235B [16] 510 / 437, [24] 527 / 474, [32] 508 / 529; 8 experts of 1024 x 512 [16] 31.8 /
+    30.8, [32] 31.7 / 35.8; Zipf-distributed routing at 16 (hot experts of 200) 482 / 472.
+
+    The others up to 16, and up to 32 where the local experts' weights exceed _STREAM_WIDE_BYTES:
+    with fewer of them HBM is no longer what takes the time and the wider items' epilogues show.
+    Mixtral bf16 [16] 473 / 452, [32] 479 / 462, [64] 502 / 512; Qwen3-30B int8 (604 MB) [24] 165 / 158,
+    [32] 167 / 166, [40] 166 / 170; bf16 128 x 1024 x 512 (402 MB) [32] 101 / 98; 201 MB: bf16 4 x 4096 x
+    2048 [16] 64.0 / 61.7, [20] 64.1 / 66.7, [32] 64.2 / 69.2, int8 128 x 1024 x 512 [24] 90.5 / 90.2, [32]
+    91.7 / 98.2; 25 MB: bf16 8 x 1024 x 512 [16] 28.7 / 27.7, [20] 28.7 / 29.7, [32] 28.7 / 32.4.
+
+    The host knows only the average.  Routing that sends every token to the same few experts makes
+    full row tiles whatever that is, and there the streaming form loses (the same DeepSeek-V3 layer,
+    64 tokens 152 / 155, 128 tokens 145 / 204, 512 tokens 288 / 447; Mixtral bf16, 128 tokens 196 / 260).
+
     ``BOLTOPS_B200_GEMM_SCHEDULE`` = ``stream`` forces it, ``tiles`` / ``pairs`` rule it out."""
     elem = 2 if kind in (_cabi.GEMM_BF16, _cabi.GEMM_F16) else 1
     if (hidden * elem) % 128 or (inter * elem) % 128:
@@ -136,11 +151,15 @@ def _use_stream(kind: int, routes: int, experts: int, hidden: int, inter: int) -
     forced = os.environ.get("BOLTOPS_B200_GEMM_SCHEDULE", "auto")
     if forced != "auto":
         return forced == "stream"
-    block = kind in (_cabi.GEMM_FP8_BLOCK, _cabi.GEMM_INT8_BLOCK)
-    return routes <= (_STREAM_MAX_AVG_ROWS_BLOCK if block else _STREAM_MAX_AVG_ROWS) * experts
+    rows = _STREAM_MAX_AVG_ROWS
+    if kind not in (_cabi.GEMM_FP8_BLOCK, _cabi.GEMM_INT8_BLOCK):
+        local = experts if local_experts is None else local_experts
+        if local * 3 * hidden * inter * elem > _STREAM_WIDE_BYTES:
+            rows = _STREAM_WIDE_MAX_AVG_ROWS
+    return routes <= rows * experts
 
 
-_STREAM_MAX_AVG_ROWS, _STREAM_MAX_AVG_ROWS_BLOCK = 32, 16
+_STREAM_MAX_AVG_ROWS, _STREAM_WIDE_MAX_AVG_ROWS, _STREAM_WIDE_BYTES = 16, 32, 256 << 20
 
 
 def gemm_schedule(kind: int, routes: int, experts: int) -> str:
@@ -384,7 +403,7 @@ def fused_experts_impl(
         args.routed_scaling_factor = float(routed_scaling_factor)
         args.out = out.data_ptr()
         args.status = ops.device_status(dev).data_ptr()
-        if _use_stream(kind, num_tokens * topk, global_num_experts, hidden, act_dim):
+        if _use_stream(kind, num_tokens * topk, global_num_experts, hidden, act_dim, e_local):
             args.schedule = _cabi.SCHEDULE_STREAM
         lib = _cabi.load()
         need = lib.bolt_moe_layer_workspace_bytes(args)
@@ -463,7 +482,8 @@ def fused_experts_impl(
                       sorted_ids=sorted_ids, sorted_weights=sorted_w, num_tokens=m, topk=topk,
                       segments=segments, num_segments=num_segments,
                       stream=segments is None and _out_peers is None
-                      and _use_stream(kind, m * topk, global_num_experts, hidden, act_dim))
+                      and _use_stream(kind, m * topk, global_num_experts, hidden, act_dim,
+                                      e_local))
 
         # ---- GEMM1 (+ activation, + re-quantisation) ---------------------------------------
         act_scale = None

@@ -296,3 +296,23 @@ def test_dense_gemm_hands_the_kernels_no_address_of_another_device(monkeypatch):
     out = torch.empty(m, n, dtype=torch.bfloat16, device="meta")
     assert gemm.gemm_a8w8_blockscale(x, w, xs, ws, out=out) is out
     assert seen[1][2] not in (0, None)      # a buffer of x's device, not the address of `out`
+
+
+def test_streaming_schedule_rule(monkeypatch):
+    """Up to 16 routes per expert; up to 32 for the kinds without block scales once the local experts
+    hold more than 256 MiB; whole 128-byte K blocks only."""
+    from boltops_b200 import _cabi
+    from boltops_b200.fused_moe import layer
+    monkeypatch.delenv("BOLTOPS_B200_GEMM_SCHEDULE", raising=False)
+
+    def limit(kind, experts, hidden, inter, local=None):
+        return max((r for r in range(1, 80)
+                    if layer._use_stream(kind, r * experts, experts, hidden, inter, local)), default=0)
+
+    assert limit(_cabi.GEMM_BF16, 8, 1024, 512) == limit(_cabi.GEMM_F16, 8, 1024, 512) == 16
+    assert limit(_cabi.GEMM_BF16, 8, 4096, 14336) == limit(_cabi.GEMM_INT8_CHANNEL, 128, 2048, 768) == 32
+    assert limit(_cabi.GEMM_INT8_CHANNEL, 128, 1024, 512) == 16
+    assert limit(_cabi.GEMM_INT8_CHANNEL, 128, 2048, 768, local=16) == 16
+    assert limit(_cabi.GEMM_FP8_CHANNEL, 64, 7168, 2048) == 32
+    assert limit(_cabi.GEMM_FP8_BLOCK, 256, 7168, 2048) == limit(_cabi.GEMM_INT8_BLOCK, 8, 1024, 512) == 16
+    assert limit(_cabi.GEMM_INT8_CHANNEL, 128, 2064, 768) == limit(_cabi.GEMM_BF16, 8, 4096, 96) == 0

@@ -598,9 +598,12 @@ def main():
     from boltops_b200.fused_moe import fused_experts, layer, ops
 
     _cabi.load()
-    config["gemm_schedule"] = layer.gemm_schedule(
-        _cabi.GEMM_BF16 if cfg["kind"] == "bf16" else _cabi.GEMM_FP8_BLOCK, m * cfg["K"] * world,
-        cfg["E"])
+    kind = {"bf16": _cabi.GEMM_BF16, "fp8_block": _cabi.GEMM_FP8_BLOCK,
+            "int8_channel": _cabi.GEMM_INT8_CHANNEL, "mxfp8": _cabi.GEMM_MXFP8,
+            "mxfp4": _cabi.GEMM_MXFP4}[cfg["kind"]]
+    # (rows that return to peers keep the layer on row tiles)
+    sizes = () if world > 1 and args.ep_direct else (cfg["H"], cfg["I"], cfg["E"] // world)
+    config["gemm_schedule"] = layer.gemm_schedule(kind, m * cfg["K"] * world, cfg["E"], *sizes)
     torch.cuda.set_device(local_rank)
     device = torch.device("cuda", local_rank)
     dist = None

@@ -106,10 +106,10 @@ def _use_tile_pairs(kind: int, routes: int, experts: int) -> bool:
     tiles), no change for per-channel 8-bit experts, and slower for the block-scaled kinds,
     whose per-K-block promotion chain now has to wait for the epilogues of two CTAs.  So pairs
     are used for bf16 / fp16 experts from three row tiles per expert on.  The host knows only
-    the average (tokens * topk / experts).  ``BOLTOPS_B200_GEMM_SCHEDULE`` = ``tiles`` /
-    ``pairs`` overrides the choice."""
+    the average (tokens * topk / experts).  ``BOLTOPS_B200_GEMM_SCHEDULE`` = ``pairs`` forces them,
+    ``tiles`` / ``stream`` rule them out."""
     forced = os.environ.get("BOLTOPS_B200_GEMM_SCHEDULE", "auto")
-    if forced == "tiles":
+    if forced in ("tiles", "stream"):
         return False
     if forced == "pairs":
         return True
@@ -144,7 +144,8 @@ def _use_stream(kind: int, routes: int, experts: int, hidden: int, inter: int,
     full row tiles whatever that is, and there the streaming form loses (the same DeepSeek-V3 layer,
     64 tokens 152 / 155, 128 tokens 145 / 204, 512 tokens 288 / 447; Mixtral bf16, 128 tokens 196 / 260).
 
-    ``BOLTOPS_B200_GEMM_SCHEDULE`` = ``stream`` forces it, ``tiles`` / ``pairs`` rule it out."""
+    ``BOLTOPS_B200_GEMM_SCHEDULE`` = ``stream`` forces it for sizes that have the form, ``tiles`` /
+    ``pairs`` rule it out."""
     elem = 2 if kind in (_cabi.GEMM_BF16, _cabi.GEMM_F16) else 1
     if (hidden * elem) % 128 or (inter * elem) % 128:
         return False
@@ -162,9 +163,18 @@ def _use_stream(kind: int, routes: int, experts: int, hidden: int, inter: int,
 _STREAM_MAX_AVG_ROWS, _STREAM_WIDE_MAX_AVG_ROWS, _STREAM_WIDE_BYTES = 16, 32, 256 << 20
 
 
-def gemm_schedule(kind: int, routes: int, experts: int) -> str:
-    """Name of the schedule ``fused_experts`` picks for this problem ("pairs" / "tiles")."""
-    return "pairs" if _use_tile_pairs(kind, routes, experts) else "tiles"
+def gemm_schedule(kind: int, routes: int, experts: int, hidden: Optional[int] = None,
+                  inter: Optional[int] = None, local_experts: Optional[int] = None) -> str:
+    """Name of the schedule ``fused_experts`` picks for this problem: "pairs", "stream" or "tiles".
+    Without the layer's sizes streaming is left out of account."""
+    if kind in (_cabi.GEMM_MXFP8, _cabi.GEMM_MXFP4):
+        return "tiles"
+    if _use_tile_pairs(kind, routes, experts):
+        return "pairs"
+    if hidden is not None and inter is not None and _use_stream(kind, routes, experts, hidden, inter,
+                                                                local_experts):
+        return "stream"
+    return "tiles"
 
 
 def _gemm_kind(w_dtype, use_fp8, use_int8, per_channel, block_shape) -> int:
@@ -481,6 +491,8 @@ def fused_experts_impl(
         common = dict(kind=kind, sorted_expert_ids=expert_ids, num_valid=num_valid,
                       sorted_ids=sorted_ids, sorted_weights=sorted_w, num_tokens=m, topk=topk,
                       segments=segments, num_segments=num_segments,
+                      # (with rows that leave for peers the form is measured on no machine yet, and
+                      # segment-scattered rows it does not have)
                       stream=segments is None and _out_peers is None
                       and _use_stream(kind, m * topk, global_num_experts, hidden, act_dim,
                                       e_local))

@@ -316,3 +316,21 @@ def test_streaming_schedule_rule(monkeypatch):
     assert limit(_cabi.GEMM_FP8_CHANNEL, 64, 7168, 2048) == 32
     assert limit(_cabi.GEMM_FP8_BLOCK, 256, 7168, 2048) == limit(_cabi.GEMM_INT8_BLOCK, 8, 1024, 512) == 16
     assert limit(_cabi.GEMM_INT8_CHANNEL, 128, 2064, 768) == limit(_cabi.GEMM_BF16, 8, 4096, 96) == 0
+
+
+def test_schedule_name_is_the_schedule(monkeypatch):
+    """What benchmarks report is what fused_experts runs, under every setting of the override."""
+    from boltops_b200 import _cabi
+    from boltops_b200.fused_moe import layer
+    monkeypatch.delenv("BOLTOPS_B200_GEMM_SCHEDULE", raising=False)
+    mixtral = (8, 4096, 14336)
+    names = [layer.gemm_schedule(_cabi.GEMM_BF16, 2 * m, *mixtral) for m in (23, 129, 8192)]
+    assert names == ["stream", "tiles", "pairs"]
+    assert layer.gemm_schedule(_cabi.GEMM_FP8_BLOCK, 96 * 8, 256, 7168, 2048) == "stream"
+    assert layer.gemm_schedule(_cabi.GEMM_FP8_BLOCK, 4096 * 8, 256, 7168, 2048) == "tiles"
+    assert layer.gemm_schedule(_cabi.GEMM_BF16, 46, 8) == "tiles"
+    for kind in (_cabi.GEMM_MXFP8, _cabi.GEMM_MXFP4):
+        assert layer.gemm_schedule(kind, 8, 64, 7168, 2048) == "tiles"
+    for forced in ("tiles", "pairs", "stream"):
+        monkeypatch.setenv("BOLTOPS_B200_GEMM_SCHEDULE", forced)
+        assert {layer.gemm_schedule(_cabi.GEMM_BF16, 2 * m, *mixtral) for m in (23, 8192)} == {forced}

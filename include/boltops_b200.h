@@ -72,7 +72,7 @@ enum bolt_gemm_kind {
   BOLT_GEMM_MXFP4 = 7         /* e4m3 rows x PACKED e2m1 weights ([E, n, k/2] bytes, low nibble
                                  first, 32-byte aligned), one E8M0 byte per 32 K elements on
                                  both operands in the same tiled layout as BOLT_GEMM_MXFP8;
-                                 plain epilogue, k a multiple of 128                        */
+                                 its epilogues, k a multiple of 128                         */
 };
 
 /* grouped-GEMM schedules */
@@ -85,8 +85,11 @@ enum bolt_gemm_schedule {
                                         BOLT_PAIR_SEGMENT_ROWS; not for the MX kind.               */
   BOLT_GEMM_SCHEDULE_STREAM = 2      /* weights streamed through small matrix instructions, only the
                                         live rows of a tile computed: for experts with a handful of
-                                        rows.  Needs sorted_ids and k in whole 128-byte blocks; rows
-                                        that pad a tile are not written; not for the MX kind, no
+                                        rows.  Needs sorted_ids and k in whole 128-byte blocks.  In
+                                        every 128-row tile the ids of tokens must come BEFORE the ids
+                                        that pad it (bolt_moe_sort_ck leaves them so): the first rows
+                                        are taken, as many as the tile has tokens.  Rows that pad a
+                                        tile are not written; not for the MX kind, no
                                         segment-scattered output.                                  */
 };
 #define BOLT_PAIR_SEGMENT_ROWS 256
@@ -508,7 +511,7 @@ typedef struct bolt_gemm_args {
      sorted order: it is the token-order matrix [a_rows >= num_tokens, k] (a_row_bytes between
      rows, a multiple of 16; 0 = dense), and sorted position p reads row sorted_ids[p] & 0xFFFFFF,
      or zeros where that id is not a token (id >= num_tokens: tile padding).  a_scale stays in
-     sorted order.  The reference gathers the same way, by pointer arithmetic inside its kernel
+     sorted order unless a_scale_token_order is set.  The reference gathers the same way, by pointer arithmetic inside its kernel
      (boltops/fused_moe/triton/moe_op.py:1479,1611-1615).                                      */
   int a_gather;
   int a_rows;
@@ -568,7 +571,11 @@ typedef struct bolt_layer_args {
   void* workspace;
   size_t workspace_bytes;
   int32_t* status;             /* optional, as in bolt_gemm_args                              */
-  int schedule;                /* enum bolt_gemm_schedule of both GEMMs: ROW_TILES or STREAM    */
+  int schedule;                /* enum bolt_gemm_schedule of both GEMMs: ROW_TILES or STREAM, the
+                                  caller's choice (equal results).  boltops_b200 streams when hidden
+                                  and inter are whole 128-byte blocks and num_tokens * topk is at most
+                                  16 * global_num_experts; for the kinds without block scales 32 times
+                                  when the local experts' weights exceed 256 MiB                */
 } bolt_layer_args;
 
 /* kernels one bolt_moe_layer call with these arguments launches (-1: invalid arguments) */

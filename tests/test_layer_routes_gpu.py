@@ -78,3 +78,46 @@ def test_dense_operands_off_the_device_or_the_16_byte_grid():
     for moved in (dict(w=w.cpu()), dict(w_scale=ws.cpu())):
         with pytest.raises(ValueError, match="x on cuda"):
             gemm_a8w8_blockscale(x.cuda(), moved.get("w", w), xs.cuda(), moved.get("w_scale", ws))
+
+
+@pytest.mark.parametrize("kind", ["mxfp8", "mxfp4"])
+@pytest.mark.parametrize("m", [1, 33, 300])          # tiles of one row, of a few, full and a remainder
+@pytest.mark.parametrize("mapped", [False, True])
+def test_mx_rows_gathered_by_the_gemm(monkeypatch, kind, m, mapped):
+    """GEMM 1 of the MX kinds reading its codes in token order or from sorted rows: the same bytes."""
+    from boltops_b200.fused_moe import fused_experts, layer, ops
+    e, topk, hidden, inter = 8, 2, 384, 256
+    g = torch.Generator().manual_seed(m)
+    x = torch.randn(m, hidden, generator=g).bfloat16().cuda()
+    wts, ids = O.make_routing(m, e, topk, 9)
+    if mapped:
+        ids[0, 1] = -1
+
+    def weight(n, k):
+        scale = torch.randint(118, 124, (e, n, k // 32), dtype=torch.uint8, generator=g).cuda()
+        if kind == "mxfp8":
+            return (torch.randn(e, n, k, generator=g) * 2).to(torch.float8_e4m3fn).cuda(), scale
+        return torch.randint(0, 256, (e, n, k // 2), dtype=torch.uint8, generator=g).cuda(), scale
+
+    (w1, s1), (w2, s2) = weight(2 * inter, hidden), weight(hidden, inter)
+    kw = dict(use_mxfp8=True) if kind == "mxfp8" else dict(use_mxfp4_w4a8=True, use_ue8m0=True)
+    if mapped:      # the upper half of the experts lives here
+        w1, s1, w2, s2 = (t[4:].contiguous() for t in (w1, s1, w2, s2))
+        kw.update(expert_map=torch.tensor([-1] * 4 + list(range(4)), dtype=torch.int32).cuda(),
+                  global_num_experts=e)
+
+    def run():
+        return fused_experts(x, w1, w2, wts.cuda(), ids.int().cuda(), w1_scale=s1, w2_scale=s2,
+                             block_shape=[1, 32], **kw).cpu()
+
+    run()       # (the weights' scales are laid out on first use)
+    outs, launches = [], []
+    for gather in (False, True):
+        monkeypatch.setattr(layer, "_GATHER", gather)
+        before = ops.launch_count()
+        outs.append(run())
+        launches.append(ops.launch_count() - before)
+        ops.check_device_status(x.device)
+    assert launches[1] == launches[0] - 1           # no sorted copy
+    assert torch.isfinite(outs[0]).all() and (m == 1 or outs[0].abs().max() > 0)
+    assert torch.equal(outs[0], outs[1])

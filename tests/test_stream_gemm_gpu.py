@@ -110,3 +110,109 @@ def test_stream_refuses_what_it_has_no_form_for():
                          b=torch.zeros(1, 64, 72, dtype=torch.bfloat16, device="cuda"), c=c,
                          sorted_expert_ids=one, num_valid=one, sorted_ids=one.repeat(128),
                          num_tokens=1, stream=True)
+
+
+def _quantised(kind, e, hidden, inter, g):
+    """Weights and keyword arguments of a layer of one kind."""
+    m1 = torch.randn(e, 2 * inter, hidden, generator=g) * 0.05
+    m2 = torch.randn(e, hidden, inter, generator=g) * 0.05
+    if kind == "bf16":
+        return m1.bfloat16().cuda(), m2.bfloat16().cuda(), {}
+    if kind == "fp8_block":
+        quant, kw = O.quantize_weight_block_fp8, dict(use_fp8_w8a8=True, block_shape=[128, 128])
+    else:
+        quant, kw = O.quantize_weight_channel_int8, dict(use_int8_w8a8=True, per_channel_quant=True)
+    (w1, s1), (w2, s2) = quant(m1), quant(m2)
+    return w1.cuda(), w2.cuda(), dict(kw, w1_scale=s1.cuda(), w2_scale=s2.cuda())
+
+
+@pytest.mark.parametrize("kind", ["bf16", "fp8_block", "int8_channel"])
+@pytest.mark.parametrize("extra", ["input_weight", "ue8m0", "not_finite"])
+def test_stream_options_equal_row_tiles(monkeypatch, kind, extra):
+    """Router weight on the input (before the gate), power-of-two scales, and rows of NaN and
+    infinity, which stay in their own rows."""
+    from boltops_b200.fused_moe import fused_experts, ops
+    if extra == "ue8m0" and kind != "fp8_block":
+        pytest.skip("power-of-two scales belong to the block-scaled kind")
+    hidden, inter, e = 512, 256, 8
+    g = torch.Generator().manual_seed(21)
+    ids = _rows(COUNTS["edges"])
+    m = ids.shape[0]
+    x = torch.randn(m, hidden, generator=g).bfloat16()
+    w1, w2, kw = _quantised(kind, e, hidden, inter, g)
+    wts = torch.rand(m, 2, generator=g)
+    bad = torch.zeros(m, dtype=torch.bool)
+    if extra == "input_weight":
+        kw["apply_router_weight_on_input"] = True
+    elif extra == "ue8m0":
+        kw["use_ue8m0"] = True
+    else:
+        bad[::7] = True
+        x[::14, 3] = float("nan")
+        x[7::14, 5] = float("inf")
+    outs = []
+    for sched in ("tiles", "stream"):
+        monkeypatch.setenv("BOLTOPS_B200_GEMM_SCHEDULE", sched)
+        out = fused_experts(x.cuda(), w1, w2, wts.cuda(), ids.cuda(), **kw)
+        ops.check_device_status(out.device)
+        outs.append(out.cpu())
+    assert torch.isfinite(outs[0][~bad]).all() and torch.equal(outs[0][~bad], outs[1][~bad])
+    assert torch.equal(outs[0].isnan(), outs[1].isnan())
+    assert torch.equal(outs[0].nan_to_num(), outs[1].nan_to_num())
+
+
+@pytest.mark.parametrize("counts", ["edges", "wide"])
+@pytest.mark.parametrize("pitch", [0, 3])               # 3: rows of the result on no 16-byte grid
+@pytest.mark.parametrize("token_scales", [False, True])
+@pytest.mark.parametrize("c_dtype", [torch.bfloat16, torch.float32])
+def test_stream_scales_by_token_and_any_row_pitch(monkeypatch, c_dtype, token_scales, pitch, counts):
+    """Row scales of the per-channel kinds in token order or in sorted order, under both schedules,
+    and results stored column by column: equal bit for bit, nothing written between the rows."""
+    from boltops_b200 import _cabi
+    from boltops_b200.fused_moe import ops
+    lib = _cabi.load()
+
+    class Lib:
+        def __getattr__(self, name):
+            return getattr(lib, name)
+
+        def bolt_grouped_gemm(self, args, stream):
+            args._obj.a_scale_token_order = int(token_scales)
+            return lib.bolt_grouped_gemm(args, stream)
+
+    ids = _rows(COUNTS[counts])
+    m, e, n, k = ids.shape[0], 8, 328, 256
+    g = torch.Generator().manual_seed(3)
+    wts = torch.rand(m, 2, generator=g).cuda()
+    sorted_ids, sorted_w, expert_ids, num_valid = ops.moe_sorting_ck(
+        ids.cuda(), wts, e, None, None, 128, None, alloc_moe_buf=False)[:4]
+    cap = sorted_ids.shape[0]
+    x = torch.randint(-127, 128, (m, k), generator=g, dtype=torch.int8).cuda()
+    w = torch.randint(-127, 128, (e, n, k), generator=g, dtype=torch.int8).cuda()
+    by_token, b_s = torch.rand(m, generator=g).cuda(), torch.rand(e, n, generator=g).cuda()
+    _, by_row = ops.gather_rows(x, sorted_ids, num_valid, cap, by_token[:, None])
+    live = (sorted_ids & 0xFFFFFF) < m
+    live[int(num_valid):] = False
+    outs = []
+    with monkeypatch.context() as patch:
+        patch.setattr(_cabi, "load", lambda: Lib())
+        for stream in (False, True):
+            buf = torch.full((cap, n + pitch), -7.0, dtype=c_dtype, device="cuda")
+            ops.grouped_gemm(kind=_cabi.GEMM_INT8_CHANNEL, epilogue=_cabi.EPI_STORE, a=x, b=w,
+                             c=buf[:, :n], sorted_expert_ids=expert_ids, num_valid=num_valid,
+                             a_scale=by_token if token_scales else by_row.reshape(-1), a_scale_ld=cap,
+                             b_scale=b_s, num_tokens=m, topk=2, mul_routed_weight=True,
+                             sorted_ids=sorted_ids, sorted_weights=sorted_w, a_gather=True, stream=stream)
+            assert (buf[:, n:] == -7.0).all()
+            outs.append(buf[live, :n].cpu())
+    ops.check_device_status(x.device)
+    token = (sorted_ids[live] & 0xFFFFFF).long().cpu()
+    expert = expert_ids.repeat_interleave(128)[:cap][live].long().cpu()
+    want = torch.einsum("rk,rnk->rn", x.cpu().double()[token], w.cpu().double()[expert])
+    want = want * by_token.cpu().double()[token][:, None] * b_s.cpu().double()[expert]
+    want = want * sorted_w[live].cpu().double()[:, None]
+    # The integer sums are exact; three products in 32 bits (2^-24 each) and, for bf16 with its eight
+    # significant bits, a rounding by half a unit in the last place (2^-8 of the value at most)
+    rel = 4 * 2.0 ** -24 + (2.0 ** -8 if c_dtype == torch.bfloat16 else 0.0)
+    assert ((outs[0].double() - want).abs() <= rel * want.abs() + 1e-30).all()
+    assert torch.equal(outs[0], outs[1])

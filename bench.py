@@ -858,7 +858,8 @@ def main():
                             frac=ach / tc_peak, traffic=traffic)
             roof.update(kernel=("k_mx_gemm (gate/up GEMM, tensor-core block scaling, activation + MX "
                                 "quantisation epilogue)" if cfg["kind"] == "mxfp8" else
-                                "k_grouped_gemm (gate/up GEMM + SiLU-mul epilogue)"),
+                                ("k_stream_gemm" if config["gemm_schedule"] == "stream"
+                                 else "k_grouped_gemm") + " (gate/up GEMM + SiLU-mul epilogue)"),
                         ms_per_launch=g_ms, algorithmic_bytes=byts, algorithmic_flops=flops,
                         tensor_time_ms=t_tc * 1e3, hbm_time_ms=t_hbm * 1e3,
                         peak_source=(peaks["source"] + " (MEASURED_PEAKS.json copy bandwidth)"

@@ -519,7 +519,7 @@ def check_device_status(device: torch.device) -> None:
     code = int(device_status(device).item())
     if code != 0:
         device_status(device).zero_()
-        raise _cabi.BoltError(f"a kernel reported an expired device-side wait (code {code}: 1-5 grouped "
+        raise _cabi.BoltError(f"a kernel reported an expired device-side wait (code {code}: 1-6 grouped "
                               f"GEMM, 20 exchange barrier, 21 exchange segment overflow)")
 
 

@@ -22,8 +22,9 @@ def gemm_a8w8_blockscale(x: torch.Tensor, w: torch.Tensor, x_scale: torch.Tensor
     """``y[m, n] = sum_kb (x[m, kb] . w[n, kb]) * x_scale[m, kb] * w_scale[n//128, kb]``.
 
     x [M, K] and w [N, K] e4m3 or int8 (same dtype), x_scale [M, K/128], w_scale
-    [N/128, K/128] floating point; K and N multiples of 128.  ``config`` / ``backend``
-    are accepted for signature compatibility and ignored (one kernel, one schedule)."""
+    [N/128, K/128] floating point; K and N multiples of 128.  w and w_scale lie on x's device;
+    x_scale and ``out`` may lie elsewhere and are copied.  ``config`` / ``backend`` are accepted
+    for signature compatibility and ignored (one kernel, one schedule)."""
     if dtype is None:
         dtype = torch.bfloat16
     if not x.is_cuda:
